@@ -153,7 +153,7 @@ def _degrees(g, structure, n, per_col):
     k = np.arange(1, 2000)
     cdf = torch.from_numpy(np.cumsum(k ** -1.5 / 2.612375348685488)).cuda()
     deg = (torch.searchsorted(cdf, _rand(g, n)) + 1).double()
-    p = torch.full_like(deg, min(1.0, per_col / 33.6))  # 33.6: the clamped law's mean
+    p = torch.full_like(deg, min(1.0, per_col / 67.9))  # 67.9: the clamped law's mean
     return torch.binomial(deg, p, generator=g).long().clamp_(min=1)
 
 
