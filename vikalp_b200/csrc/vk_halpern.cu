@@ -36,6 +36,7 @@
 // tolerance, the iterates move to float64 and the float64 engine finishes
 // (the polish). The answer is always checked in float64.
 #include "vk_engine.cuh"
+#include "vk_halpern_resident.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -47,43 +48,8 @@ namespace {
 
 constexpr int kRuizPasses = 10;
 constexpr int kPowerMax = 200;
-constexpr int kColCheckSums = 2;       // |x^-x|^2, |x^-x0|^2
-constexpr int kRowCheckSums = 2;       // |y^-y|^2, |y^-y0|^2
-constexpr int kKktRowSums = 3;         // primal res^2, dual-obj rows, row-dual violations^2
-constexpr int kKktColSums = 5;         // dual res^2, dual-obj cols, primal obj, box violation^2, x'Qx
+constexpr int kRsIterations = 1024; // iterations in one launch of the resident kernel
 constexpr int64_t kTunePassesMinNnz = 2000000; // per-pass variant tuning from this many nonzeros
-
-struct HalCtl {
-    double eta, omega, tau, sigma;
-    double r_restart, r_prev;
-    double rel_p, rel_d, rel_gap, kkt;
-    double bnorm, cnorm, offset, tol;
-    double knorm, lq, rho, pad_d; // sigma_max(K), lambda_max(Q^) (0: LP), reflection
-    double theta, freeze;                   // primal-weight smoothing; no update below this KKT
-    double beta_suff, beta_nec, beta_art;   // restart thresholds
-    long long k_base, total, limit, restarts, checks;
-    int done, status, restart_now, pad;
-};
-
-// Step sizes for primal weight omega: tau = eta/omega, sigma = eta*omega.
-// LP (lq == 0): eta = 0.99/|K| and full reflection rho = 1. QP: the explicit
-// gradient step on 0.5 x'Q^x needs 1/tau - sigma |K|^2 >= L; eta solves
-// tau L + eta^2 |K|^2 = 0.99^2 and the reflection is cut to
-// rho = 0.99 (1 - 1/(2 kappa)), kappa = (1/tau - sigma |K|^2) / L, which keeps
-// (1+rho) T - rho I nonexpansive (Condat's bound on the relaxation of the
-// primal-dual iteration with a smooth term).
-__host__ __device__ inline void step_params(double knorm, double lq, double omega, double &eta, double &rho) {
-    if (!(lq > 0.0)) {
-        eta = knorm > 0.0 ? 0.99 / knorm : 1.0;
-        rho = 1.0;
-        return;
-    }
-    const double k2 = knorm * knorm, b = lq / omega, c = 0.9801;
-    eta = 2.0 * c / (b + sqrt(b * b + 4.0 * k2 * c));
-    const double tau = eta / omega;
-    const double kappa = (1.0 - eta * eta * k2) / (tau * lq);
-    rho = fmin(1.0, 0.99 * (1.0 - 1.0 / (2.0 * kappa)));
-}
 
 // ---- scaling (FP64, original values) -----------------------------------------
 
@@ -271,18 +237,8 @@ struct KktRowEpi : EpiBase<T> {
     __device__ bool skip() const { return ctl->done != 0; }
     __device__ Pre load(int i) const { return Pre{yhat[i], rl[i], ru[i], rs[i]}; }
     __device__ void row_pre(int, const T (&s)[1], const Pre &p, double (&red)[NR]) const {
-        const double a = static_cast<double>(s[0]);
-        const double lo = static_cast<double>(p.rl), hi = static_cast<double>(p.ru), r = static_cast<double>(p.r);
-        const double pr = (a - clampbox(a, lo, hi)) / r;
-        red[0] += pr * pr;
-        const double y = static_cast<double>(p.y);
-        const double yl = smax(0.0, -y), yu = smax(0.0, y);
-        if (yl > 0.0) {
-            if (isfinite(lo)) red[1] += lo * yl; else red[2] += (r * yl) * (r * yl);
-        }
-        if (yu > 0.0) {
-            if (isfinite(hi)) red[1] -= hi * yu; else red[2] += (r * yu) * (r * yu);
-        }
+        kkt_row_terms(static_cast<double>(s[0]), static_cast<double>(p.rl), static_cast<double>(p.ru),
+                      static_cast<double>(p.r), static_cast<double>(p.y), red);
     }
     __device__ void finish(double (&red)[NR], double *scratch, int block) const {
         block_sum<NR>(red, scratch);
@@ -305,21 +261,9 @@ struct KktColEpi : EpiBase<T> {
     __device__ bool skip() const { return ctl->done != 0; }
     __device__ Pre load(int j) const { return Pre{xhat[j], c[j], l[j], u[j], cs[j], qx ? qx[j] : T(0)}; }
     __device__ void row_pre(int, const T (&s)[1], const Pre &p, double (&red)[NR]) const {
-        const double q = static_cast<double>(p.q);
-        const double lam = static_cast<double>(p.c) + q + static_cast<double>(s[0]);
-        const double d = static_cast<double>(p.d);
-        const double lo = static_cast<double>(p.l), hi = static_cast<double>(p.u), x = static_cast<double>(p.x);
-        const double vl = smax(0.0, lam), vu = smax(0.0, -lam);
-        if (vl > 0.0) {
-            if (isfinite(lo)) red[1] += lo * vl; else red[0] += (vl / d) * (vl / d);
-        }
-        if (vu > 0.0) {
-            if (isfinite(hi)) red[1] -= hi * vu; else red[0] += (vu / d) * (vu / d);
-        }
-        red[2] += static_cast<double>(p.c) * x;
-        const double bx = (x - clampbox(x, lo, hi)) * d;
-        red[3] += bx * bx;
-        red[4] += x * q;
+        kkt_col_terms(static_cast<double>(s[0]), static_cast<double>(p.c), static_cast<double>(p.q),
+                      static_cast<double>(p.d), static_cast<double>(p.l), static_cast<double>(p.u),
+                      static_cast<double>(p.x), red);
     }
     __device__ void finish(double (&red)[NR], double *scratch, int block) const {
         block_sum<NR>(red, scratch);
@@ -368,7 +312,7 @@ __global__ void __launch_bounds__(kControlThreads)
     if (threadIdx.x == 0) skip = ctl->done;
     __syncthreads();
     if (skip) return;
-    double s[kColCheckSums + kRowCheckSums + kKktRowSums + kKktColSums];
+    double s[kCheckSums];
     int o = 0;
     for (int r = 0; r < kColCheckSums; ++r) s[o++] = block_reduce_range(pc, g.col, kColCheckSums, r, scratch);
     for (int r = 0; r < kRowCheckSums; ++r) s[o++] = block_reduce_range(pr, g.row, kRowCheckSums, r, scratch);
@@ -376,53 +320,7 @@ __global__ void __launch_bounds__(kControlThreads)
     for (int r = 0; r < kKktColSums; ++r) s[o++] = block_reduce_range(pkc, g.kkt_col, kKktColSums, r, scratch);
     if (threadIdx.x != 0) return;
     HalCtl c = *ctl;
-    const double dx2 = s[0], dx0 = s[1], dy2 = s[2], dy0 = s[3];
-    const double rp2 = s[4], dobj_r = s[5], viol2 = s[6];
-    const double rd2 = s[7], dobj_c = s[8], box2 = s[10], quad = s[11];
-    const double pobj = s[9] + 0.5 * quad + c.offset;
-    const double dobj = dobj_r + dobj_c - 0.5 * quad + c.offset;
-    c.total += chunk;
-    c.checks += 1;
-    c.rel_p = (sqrt(rp2) + sqrt(box2)) / (1.0 + c.bnorm);
-    c.rel_d = sqrt(rd2 + viol2) / (1.0 + c.cnorm);
-    c.rel_gap = fabs(pobj - dobj) / (1.0 + fabs(pobj) + fabs(dobj));
-    c.kkt = smax(smax(c.rel_p, c.rel_d), c.rel_gap);
-    c.restart_now = 0;
-    if (!(c.kkt == c.kkt)) { // NaN: stop, the host reports a numerical failure
-        c.done = 1;
-        c.status = VK_STATUS_NUMERICAL_FAILURE;
-    } else if (c.kkt <= c.tol) {
-        c.done = 1;
-        c.status = VK_STATUS_OPTIMAL;
-    } else if (c.total >= c.limit) {
-        c.done = 1;
-        c.status = VK_STATUS_ITERATION_LIMIT;
-    } else {
-        const double r = sqrt(c.omega * dx2 + dy2 / c.omega);
-        const long long k = c.k_base + chunk;
-        bool restart = false;
-        if (c.r_restart < 0.0) {
-            c.r_restart = r;
-        } else {
-            restart = (r <= c.beta_suff * c.r_restart) || (r <= c.beta_nec * c.r_restart && r > c.r_prev) ||
-                      (static_cast<double>(k) >= c.beta_art * static_cast<double>(c.total));
-        }
-        c.r_prev = r;
-        if (restart) {
-            const double mx = sqrt(dx0), my = sqrt(dy0);
-            if (mx > 1e-10 && my > 1e-10 && c.theta > 0.0 && c.kkt >= c.freeze)
-                c.omega = exp(c.theta * log(my / mx) + (1.0 - c.theta) * log(c.omega));
-            step_params(c.knorm, c.lq, c.omega, c.eta, c.rho);
-            c.tau = c.eta / c.omega;
-            c.sigma = c.eta * c.omega;
-            c.k_base = 0;
-            c.restarts += 1;
-            c.restart_now = 1;
-            c.r_restart = r;
-        } else {
-            c.k_base = k;
-        }
-    }
+    halpern_decide(c, s, chunk);
     *ctl = c;
 }
 
@@ -504,6 +402,14 @@ struct HalState {
     DevBuf<T> q, qx;                        // QP: Q^ = D Q D values, Q^ x
 };
 
+// The resident launch of one precision, when the model fits (plan_resident).
+struct Resident {
+    bool on = false, small = false; // small: 16-bit indices
+    int grid = 0, threads = 0;
+    size_t smem = 0;
+    int cap_a = 0, cap_t = 0, cap_q = 0, rows = 0, cols = 0;
+};
+
 class HalpernEngine final : public Engine {
 public:
     HalpernEngine(const DeviceModel &dm, const vk_options &o, cudaStream_t s) : dm_(dm), o_(o), s_(s) {
@@ -528,6 +434,7 @@ public:
         pr_.reset(static_cast<size_t>(kMaxGrid) * kRowCheckSums);
         pkr_.reset(static_cast<size_t>(kMaxGrid) * kKktRowSums);
         pkc_.reset(static_cast<size_t>(kMaxGrid) * kKktColSums);
+        plan_resident();
     }
 
     ~HalpernEngine() override {
@@ -640,7 +547,7 @@ public:
         bool confirmed = false; // mixed: the float32 answer passed the float64 evaluation
         if (mixed_) {
             copy_state<float, double>(s64_, s32_);
-            if (!g32_) g32_ = capture(s32_);
+            if (!rs32_.on && !g32_) g32_ = capture(s32_);
             // float32 phase. When its own (float32) KKT evaluation reaches the
             // tolerance, the point is evaluated again in float64 with no
             // float64 iteration: accepted there, the solve ends; otherwise the
@@ -662,7 +569,7 @@ public:
                     timed_out = true;
                     break;
                 }
-                poll_chunk(g32_);
+                advance(s32_, rs32_, g32_);
                 HalCtl h = hctl_[0];
                 if (h.done) {
                     if (h.status != VK_STATUS_OPTIMAL) break;
@@ -720,13 +627,13 @@ public:
             }
         }
         if (!timed_out && !confirmed) {
-            if (!g64_) g64_ = capture(s64_);
+            if (!rs64_.on && !g64_) g64_ = capture(s64_);
             for (;;) {
                 if (over_time(started)) {
                     timed_out = true;
                     break;
                 }
-                poll_chunk(g64_);
+                advance(s64_, rs64_, g64_);
                 if (hctl_[0].done) break;
             }
         }
@@ -759,7 +666,7 @@ public:
 
 private:
     // Writes a control block to the device from the pinned host copy (later
-    // reads of it on the stream, poll_chunk's included, are ordered after).
+    // reads of it on the stream, advance's included, are ordered after).
     void put_control(const HalCtl &h) {
         hctl_[0] = h;
         VK_CUDA(cudaMemcpyAsync(ctl_.get(), hctl_.get(), sizeof(HalCtl), cudaMemcpyHostToDevice, s_));
@@ -791,9 +698,19 @@ private:
         return std::isfinite(o_.time_limit_seconds) && seconds_since(t0) >= o_.time_limit_seconds;
     }
 
-    void poll_chunk(cudaGraphExec_t g) {
-        VK_CUDA(cudaGraphLaunch(g, s_));
-        launches_ += graph_nodes_;
+    // The next check interval (several in one launch of the float64 resident
+    // kernel: it stops by itself; the float32 phase's plateau rule wants every
+    // check, as does the trace), and the control block back on the host.
+    template <class T>
+    void advance(HalState<T> &st, const Resident &r, cudaGraphExec_t g) {
+        if (r.on) {
+            const bool every = sizeof(T) == 4 || o_.verbose >= 2;
+            launch_resident(st, r, every ? 1 : std::max(1, kRsIterations / chunk_));
+            launches_ += 1;
+        } else {
+            VK_CUDA(cudaGraphLaunch(g, s_));
+            launches_ += graph_nodes_;
+        }
         VK_CUDA(cudaMemcpyAsync(hctl_.get(), ctl_.get(), sizeof(HalCtl), cudaMemcpyDeviceToHost, s_));
         VK_CUDA(cudaStreamSynchronize(s_));
         check_device_error(s_);
@@ -802,6 +719,107 @@ private:
             std::fprintf(stderr, "[vikalp_b200] halpern %lld kkt %.3e p %.2e d %.2e gap %.2e omega %.4g restarts %lld\n",
                          h.total, h.kkt, h.rel_p, h.rel_d, h.rel_gap, h.omega / omega0_, h.restarts);
         }
+    }
+
+    // A model whose matrices fit the GPU's shared memory iterates there
+    // (vk_resident.cuh). A pinned kernel variant keeps the passes.
+    void plan_resident() {
+        if (dm_.m == 0 || dm_.nnz == 0 || forced_variant() >= 0) return;
+        const int64_t nnz = 2 * dm_.nnz + (dm_.qp ? dm_.q_nnz : 0);
+        if (nnz * static_cast<int64_t>(sizeof(float) + 2) > static_cast<int64_t>(kRsMaxGrid) * kRsSmem) return;
+        const int m = dm_.m, n = dm_.n;
+        std::vector<int> ro(m + 1), rot(n + 1), roq(dm_.qp ? n + 1 : 0);
+        const auto get = [&](std::vector<int> &h, const DevBuf<int> &d) {
+            if (!h.empty())
+                VK_CUDA(cudaMemcpyAsync(h.data(), d.get(), h.size() * sizeof(int), cudaMemcpyDeviceToHost, s_));
+        };
+        get(ro, dm_.a.ro);
+        get(rot, dm_.at.ro);
+        get(roq, dm_.q.ro);
+        VK_CUDA(cudaStreamSynchronize(s_));
+        Resident r;
+        r.grid = rs_grid(dm_.nnz);
+        r.threads = rs_threads(dm_.nnz, r.grid);
+        r.small = m <= 65536 && n <= 65536;
+        // columns are split by their nonzeros in A and Q together
+        std::vector<int> both(rot);
+        for (size_t j = 0; j < roq.size(); ++j) both[j] += roq[j];
+        const RsPart pa = rs_partition(ro, m, r.grid), pt = rs_partition(both, n, r.grid);
+        r.rows = pa.rows;
+        r.cols = pt.rows;
+        r.cap_a = static_cast<int>(pa.nnz);
+        for (int b = 0; b < r.grid; ++b) {
+            r.cap_t = std::max(r.cap_t, rot[pt.at[b + 1]] - rot[pt.at[b]]);
+            if (dm_.qp) r.cap_q = std::max(r.cap_q, roq[pt.at[b + 1]] - roq[pt.at[b]]);
+        }
+        rs64_ = rs32_ = r;
+        plan_one<double>(rs64_);
+        if (mixed_) plan_one<float>(rs32_);
+        if (!rs64_.on && !rs32_.on) return;
+        part_a_.reset(pa.at.size());
+        part_t_.reset(pt.at.size());
+        counter_.reset(1);
+        partials_.reset(static_cast<size_t>(kRsMaxGrid) * kCheckSums);
+        VK_CUDA(cudaMemcpyAsync(part_a_.get(), pa.at.data(), part_a_.bytes(), cudaMemcpyHostToDevice, s_));
+        VK_CUDA(cudaMemcpyAsync(part_t_.get(), pt.at.data(), part_t_.bytes(), cudaMemcpyHostToDevice, s_));
+        VK_CUDA(cudaStreamSynchronize(s_));
+    }
+    template <class T>
+    void plan_one(Resident &r) {
+        with_kernel<T>(r, [&](auto kernel, auto index) {
+            r.smem = RsHalLayout<T, decltype(index)>(r.cap_a, r.cap_t, r.cap_q, r.rows, r.cols, dm_.qp).bytes;
+            r.on = rs_fits(kernel, r.grid, r.threads, r.smem);
+        });
+    }
+    // f(kernel, a value of its index type)
+    template <class T, class F>
+    void with_kernel(const Resident &r, F &&f) {
+        if (dm_.qp)
+            r.small ? f(rs_halpern_kernel<T, uint16_t, true>, uint16_t()) : f(rs_halpern_kernel<T, int, true>, int());
+        else
+            r.small ? f(rs_halpern_kernel<T, uint16_t, false>, uint16_t()) : f(rs_halpern_kernel<T, int, false>, int());
+    }
+    template <class T>
+    void launch_resident(HalState<T> &st, const Resident &r, int chunks) {
+        RsHalArgs<T> a{};
+        a.ro_a = dm_.a.ro.get();
+        a.ci_a = dm_.a.ci.get();
+        a.ro_t = dm_.at.ro.get();
+        a.ci_t = dm_.at.ci.get();
+        a.ro_q = dm_.q.ro.get();
+        a.ci_q = dm_.q.ci.get();
+        a.va = st.ka.get();
+        a.vt = st.kat.get();
+        a.vq = st.q.get();
+        a.part_a = part_a_.get();
+        a.part_t = part_t_.get();
+        a.cap_a = r.cap_a;
+        a.cap_t = r.cap_t;
+        a.cap_q = r.cap_q;
+        a.rows = r.rows;
+        a.cols = r.cols;
+        a.x = st.x.get();
+        a.x0 = st.x0.get();
+        a.xbar = st.xbar.get();
+        a.xhat = st.xhat.get();
+        a.y = st.y.get();
+        a.y0 = st.y0.get();
+        a.yhat = st.yhat.get();
+        a.c = st.c.get();
+        a.l = st.l.get();
+        a.u = st.u.get();
+        a.cs = st.cs.get();
+        a.rl = st.rl.get();
+        a.ru = st.ru.get();
+        a.rs = st.rs.get();
+        a.ctl = ctl_.get();
+        a.partials = partials_.get();
+        a.counter = counter_.get();
+        a.err = device_error_flag();
+        a.chunk = chunk_;
+        a.chunks = chunks;
+        VK_CUDA(cudaMemsetAsync(counter_.get(), 0, sizeof(unsigned), s_));
+        with_kernel<T>(r, [&](auto kernel, auto) { rs_launch(kernel, r.grid, r.threads, r.smem, s_, a); });
     }
 
     // Ruiz (infinity norm) passes, then one Pock-Chambolle (alpha = 1) pass.
@@ -1114,6 +1132,10 @@ private:
     double knorm_ = 0.0, lq_ = 0.0, omega0_ = 1.0, bnorm_ = 0.0, cnorm_ = 0.0;
     cudaGraphExec_t g64_ = nullptr, g32_ = nullptr;
     long long graph_nodes_ = 0, launches_ = 0;
+    Resident rs64_, rs32_;
+    DevBuf<int> part_a_, part_t_;
+    DevBuf<unsigned> counter_;
+    DevBuf<double> partials_;
     bool tuned_ = false;
     int col_var_[2] = {-1, -1}, row_var_[2] = {-1, -1}; // tuned pass variants [float64, float32]
 };

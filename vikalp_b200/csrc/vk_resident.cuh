@@ -1,0 +1,215 @@
+// Resident iterations: an LP (or QP) whose matrices fit the GPU's shared memory
+// iterates in one cooperative launch.
+//
+// A pass over a matrix of up to a million nonzeros is latency, not bandwidth:
+// launch, row offsets -> column index -> gathered value through L2, epilogue,
+// next launch. Here every CTA (one per SM) keeps its contiguous range of rows
+// of A and of columns (rows of A') in shared memory for the whole launch --
+// values, indices, bounds, iterates -- and only the two gathered vectors go
+// through L2: a pass gathers, multiplies, sums its rows and writes its own
+// slice of the other vector, and one grid barrier orders the passes. The
+// gathers are taken nonzero by nonzero (every thread the same number in
+// flight, whatever the row lengths), the products staged in shared memory and
+// the row sums taken from there.
+//
+// The grid barrier spins on a counter in L2 (2,550 cycles with 148 CTAs;
+// flags polled by every CTA and a two-level tree took 4,300-7,300, and packets
+// of value and iteration number, which need no barrier, no less than it once
+// their lines are shared by many readers). The launch is cooperative, so all
+// CTAs are resident; the spin is bounded, and a CTA that gives up records the
+// timeout in the device error flag and leaves, as the others then do.
+#pragma once
+
+#include "vk_csr.cuh"
+
+namespace vk {
+
+constexpr int kRsThreads = 768;     // threads of a CTA, at most
+constexpr int kRsSmem = 220 * 1024; // dynamic shared memory of a CTA (227 KB less the static part)
+constexpr int kRsRowCost = 4;       // partition: a row costs this many nonzeros
+constexpr int kRsGather = 4;        // gathers in flight per thread
+constexpr int kRsWarpRow = 32;      // a row of more than this many products per lane goes to a whole warp
+constexpr int kRsMaxGrid = 160;
+constexpr unsigned kRsPolls = 1u << 25; // over ten seconds
+
+// Rows [part[b], part[b+1]) of a matrix belong to CTA b; the largest shares.
+struct RsPart {
+    int rows = 0;
+    int64_t nnz = 0;
+    std::vector<int> at;
+};
+
+// ---- device side ----------------------------------------------------------------
+
+// One CTA's share of a matrix, in shared memory.
+template <class T, class I>
+struct RsSide {
+    const T *v;
+    const I *idx;
+    const int *ro;
+    int rows, nnz, L;
+};
+
+template <class T, class I>
+__device__ RsSide<T, I> rs_load(const int *__restrict__ ro, const int *__restrict__ ci, const T *__restrict__ val,
+                                int r0, int r1, T *v, I *idx, int *sro) {
+    const int k0 = ro[r0], nnz = ro[r1] - k0, rows = r1 - r0;
+    for (int k = threadIdx.x; k < nnz; k += blockDim.x) {
+        v[k] = __ldg(val + k0 + k);
+        idx[k] = static_cast<I>(__ldg(ci + k0 + k));
+    }
+    for (int r = threadIdx.x; r <= rows; r += blockDim.x) sro[r] = ro[r0 + r] - k0;
+    // lanes per row: every thread busy in one round, at most about one per nonzero
+    int L = 1;
+    while (L < 32 && rows * L * 2 <= static_cast<int>(blockDim.x) && rows * L < nnz) L *= 2;
+    return RsSide<T, I>{v, idx, sro, rows, nnz, L};
+}
+
+// prod[k] = v_k x[idx_k]; x is written by other CTAs during the launch. A:
+// the products' type (float64 in the checks).
+template <class A, class T, class I>
+__device__ __forceinline__ void rs_products(const RsSide<T, I> &s, const T *x, A *prod) {
+    const int nt = blockDim.x;
+    int k = threadIdx.x;
+    for (; k + (kRsGather - 1) * nt < s.nnz; k += kRsGather * nt) {
+        T g[kRsGather];
+#pragma unroll
+        for (int u = 0; u < kRsGather; ++u) g[u] = __ldcg(x + s.idx[k + u * nt]);
+#pragma unroll
+        for (int u = 0; u < kRsGather; ++u)
+            prod[k + u * nt] = static_cast<A>(s.v[k + u * nt]) * static_cast<A>(g[u]);
+    }
+    if (k < s.nnz) { // fewer than kRsGather left
+        T g[kRsGather];
+#pragma unroll
+        for (int u = 0; u < kRsGather; ++u)
+            if (k + u * nt < s.nnz) g[u] = __ldcg(x + s.idx[k + u * nt]);
+#pragma unroll
+        for (int u = 0; u < kRsGather; ++u)
+            if (k + u * nt < s.nnz) prod[k + u * nt] = static_cast<A>(s.v[k + u * nt]) * static_cast<A>(g[u]);
+    }
+}
+
+// row(r, sum) for every row, in one lane of the row's group.
+template <class A, class T, class I, class F>
+__device__ __forceinline__ void rs_rows(const RsSide<T, I> &s, const A *prod, F &&row) {
+    const unsigned FULL = 0xffffffffu;
+    const int L = s.L, lane = threadIdx.x & 31, sl = lane & (L - 1);
+    const int first = (static_cast<int>(threadIdx.x) & ~31) / L; // the warp's first row: uniform trip count
+    for (int rb = first; rb < s.rows; rb += static_cast<int>(blockDim.x) / L) {
+        const int r = rb + lane / L;
+        const bool valid = r < s.rows;
+        const int a = valid ? s.ro[r] : 0, b = valid ? s.ro[r + 1] : 0;
+        const bool lone = b - a > kRsWarpRow * L; // summed by the whole warp below
+        A acc = A(0);
+        if (!lone)
+            for (int k = a + sl; k < b; k += L) acc += prod[k];
+        for (int o = L >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(FULL, acc, o);
+        unsigned lm = __ballot_sync(FULL, lone && sl == 0);
+        while (lm) {
+            const int src = __ffs(lm) - 1;
+            const int fa = __shfl_sync(FULL, a, src), fb = __shfl_sync(FULL, b, src);
+            A part = A(0);
+            for (int k = fa + lane; k < fb; k += 32) part += prod[k];
+            part = warp_sum(part);
+            if (lane == src) acc = part;
+            lm &= lm - 1u;
+        }
+        if (valid && sl == 0) row(r, acc);
+    }
+}
+
+// A CTA's block barrier at the end of a gather: false when any of its threads
+// gave up (`ok` false), after recording that.
+__device__ __forceinline__ bool rs_block(bool ok, int *err) {
+    if (!ok) atomicCAS(err, 0, static_cast<int>(kDevErrBarrierTimeout));
+    return __syncthreads_or(!ok) == 0;
+}
+
+// Grid barrier over the gridDim.x CTAs of a cooperative launch; `counter` is
+// zero at the launch. All writes before it are visible after it.
+struct RsBarrier {
+    unsigned *counter;
+    int *err;
+    unsigned target = 0;
+
+    // False when another CTA never came: the caller returns.
+    __device__ __forceinline__ bool sync() {
+        __syncthreads();
+        target += gridDim.x;
+        bool ok = true;
+        if (threadIdx.x == 0) {
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
+            unsigned now = 0, polls = 0;
+            do {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(counter) : "memory");
+            } while (static_cast<int>(now - target) < 0 && ++polls < kRsPolls);
+            ok = static_cast<int>(now - target) >= 0;
+        }
+        return rs_block(ok, err);
+    }
+};
+
+// Sums v over the grid in CTA order: out[r] (shared memory) holds the totals
+// after it, in every CTA. `partials`: kRsMaxGrid * NR doubles in global memory.
+template <int NR>
+__device__ __forceinline__ bool rs_sum(double (&v)[NR], double *partials, double *scratch, double *out, RsBarrier &bar) {
+    block_sum<NR>(v, scratch);
+    if (threadIdx.x == 0)
+        for (int r = 0; r < NR; ++r) partials[static_cast<size_t>(blockIdx.x) * NR + r] = v[r];
+    if (!bar.sync()) return false;
+    const int lane = threadIdx.x & 31;
+    for (int r = static_cast<int>(threadIdx.x) >> 5; r < NR; r += static_cast<int>(blockDim.x) / 32) {
+        double t = 0.0;
+        for (int b = lane; b < static_cast<int>(gridDim.x); b += 32) t += __ldcg(partials + static_cast<size_t>(b) * NR + r);
+        t = warp_sum(t);
+        if (lane == 0) out[r] = t;
+    }
+    __syncthreads();
+    return true;
+}
+
+// ---- host side (vk_resident.cu) ------------------------------------------------------
+
+// Splits `rows` rows over `ctas` shares of about equal cost.
+RsPart rs_partition(const std::vector<int> &ro, int rows, int ctas);
+
+// CTAs (at most one per SM) and threads for `nnz` nonzeros. Timed per
+// iteration (float64 Halpern, 37 / 74 / 148 CTAs x 256 / 512 / 768 / 1024
+// threads): 4,000 nonzeros 4.8 us with 37 x 256 (148 x 1024: 5.3), 40,000
+// nonzeros 5.4 us with 148 x 256 (37 x 256: 6.5, 148 x 1024: 5.8), 120,000
+// nonzeros 6.4 us with 148 x 512 (256: 7.3, 1024: 6.8), 600,000 nonzeros 11.0
+// us with 148 x 768 (256: 13.5, 1024: 11.5).
+int rs_grid(int64_t nnz);
+int rs_threads(int64_t nnz, int grid);
+
+template <class K, class... A>
+inline void rs_launch(K kernel, int grid, int threads, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(grid));
+    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    VK_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+}
+
+// True when `grid` CTAs of `kernel` are resident at once with `smem` bytes of
+// dynamic shared memory each (also sets the kernel's shared-memory limit).
+template <class K>
+inline bool rs_fits(K kernel, int grid, int threads, size_t smem) {
+    if (smem > static_cast<size_t>(kRsSmem)) return false;
+    int dev = 0, sms = 0, per = 0, coop = 0;
+    VK_CUDA(cudaGetDevice(&dev));
+    VK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    VK_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    VK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRsSmem));
+    VK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem));
+    return coop != 0 && grid <= per * sms;
+}
+
+} // namespace vk
