@@ -19,7 +19,7 @@
 // F), M'u a pass over A (gathers u, masks by R) -- the same fused sparse-pass
 // kernels as the solver, with the LSQR vector updates in their epilogues and
 // per-tile partial sums reduced per instance in a fixed order. The scalar
-// recurrences run on the device, one thread per instance; a chunk of
+// recurrences run on the device, one warp per instance; a chunk of
 // iterations is one CUDA graph.
 #include "vk_blockdiag.cuh"
 #include "vk_engine.cuh"
@@ -89,10 +89,11 @@ __global__ void segment_norm2_kernel(const double *__restrict__ a, const int *__
     if (lane == 0) out[b] = s;
 }
 
+// Sum of an instance's per-tile partials over the lanes of its warp (fixed order).
 __device__ double tile_sum(const double *p, int t0, int t1) {
     double s = 0.0;
-    for (int t = t0; t < t1; ++t) s += p[t];
-    return s;
+    for (int t = t0 + (static_cast<int>(threadIdx.x) & 31); t < t1; t += 32) s += p[t];
+    return warp_sum(s);
 }
 
 // Start: beta_1 = |F g|; alpha = 1 and v = 0 so the first A pass gives
@@ -116,9 +117,10 @@ __global__ void lsqr_start_kernel(LsqrCtl c, const double *nrm2) {
 // The first alpha: alpha_1 = |M'u_1|; phibar = beta_1, rhobar = alpha_1,
 // and the search direction starts at v_1 (t1 = 0, t2 = 0 in the update kernel).
 __global__ void lsqr_first_alpha_kernel(LsqrCtl c) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (b >= c.count || c.done[b]) return;
     const double alpha = sqrt(tile_sum(c.pa, c.tbeg_a[b], c.tbeg_a[b + 1]));
+    if ((threadIdx.x & 31) != 0) return;
     c.alpha[b] = alpha;
     c.phibar[b] = c.beta[b];
     c.rhobar[b] = alpha;
@@ -163,13 +165,15 @@ struct AdjColEpi : EpiBase<double> {
 // beta <- |u|; a finished instance (stop set by the previous alpha step) is
 // marked done here, after its last search-direction update.
 __global__ void lsqr_beta_kernel(LsqrCtl c) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (b >= c.count || c.done[b]) return;
+    const bool lead = (threadIdx.x & 31) == 0;
     if (c.stop[b]) {
-        c.done[b] = 1;
+        if (lead) c.done[b] = 1;
         return;
     }
-    c.beta[b] = sqrt(tile_sum(c.pat, c.tbeg_at[b], c.tbeg_at[b + 1]));
+    const double beta = sqrt(tile_sum(c.pat, c.tbeg_at[b], c.tbeg_at[b + 1]));
+    if (lead) c.beta[b] = beta;
 }
 
 // A pass (rows i, gathers ubar): v <- R (M'u) - beta v with u = ubar / beta
@@ -204,9 +208,10 @@ struct AdjRowEpi : EpiBase<double> {
 // alpha <- |v|, then the plane rotation of LSQR and its stopping tests:
 // |r| <= tol |g_F| (consistent system) or |M'r| <= tol |M|_F |r| (least squares).
 __global__ void lsqr_alpha_kernel(LsqrCtl c) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (b >= c.count || c.done[b] || c.stop[b]) return;
     const double alpha = sqrt(tile_sum(c.pa, c.tbeg_a[b], c.tbeg_a[b + 1]));
+    if ((threadIdx.x & 31) != 0) return;
     const double beta = c.beta[b];
     const double rhobar = c.rhobar[b], phibar = c.phibar[b];
     const double rho = hypot(rhobar, beta);
@@ -332,7 +337,7 @@ public:
         // v_1 = M'u_1 / beta_1, alpha_1 = |v_1|, d_1 = v_1
         if (m > 0) {
             row_pass(c);
-            lsqr_first_alpha_kernel<<<ceil_div(B, 128), 128, 0, s_>>>(c);
+            lsqr_first_alpha_kernel<<<ceil_div(int64_t(B) * 32, 128), 128, 0, s_>>>(c);
             lsqr_update_kernel<<<grid1d(m), 256, 0, s_>>>(c, d_.rinst.get(), vbar_.get(), w_.get(), dir_.get(), m);
             VK_LAUNCH_CHECK();
         }
@@ -442,9 +447,9 @@ private:
         VK_CUDA(cudaStreamBeginCapture(s_, cudaStreamCaptureModeThreadLocal));
         for (int it = 0; it < kAdjChunk; ++it) {
             col_pass(c);
-            lsqr_beta_kernel<<<ceil_div(B_, 128), 128, 0, s_>>>(c);
+            lsqr_beta_kernel<<<ceil_div(int64_t(B_) * 32, 128), 128, 0, s_>>>(c);
             row_pass(c);
-            lsqr_alpha_kernel<<<ceil_div(B_, 128), 128, 0, s_>>>(c);
+            lsqr_alpha_kernel<<<ceil_div(int64_t(B_) * 32, 128), 128, 0, s_>>>(c);
             lsqr_update_kernel<<<grid1d(m), 256, 0, s_>>>(c, d_.rinst.get(), vbar_.get(), w_.get(), dir_.get(), m);
             VK_LAUNCH_CHECK();
         }

@@ -134,16 +134,17 @@ __global__ void gather_values_kernel(const int *__restrict__ perm, const TS *__r
         dst[t] = static_cast<TD>(src[perm[t]]);
 }
 
-// chunks[c] = first row r with cost(r) >= c * kChunkCost, cost(r) = ro[r] +
+// chunks[c] = first row r with cost(r) >= c * cost, cost(r) = ro[r] +
 // kRowCost * r (monotone); chunks[nchunks] = rows. Thread per r in [0, rows].
-__global__ void chunk_rows_kernel(const int *__restrict__ ro, int rows, int nchunks, int *__restrict__ chunks) {
+__global__ void chunk_rows_kernel(const int *__restrict__ ro, int rows, int cost, int nchunks,
+                                  int *__restrict__ chunks) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r > rows) return;
     const int64_t hi = static_cast<int64_t>(ro[r]) + static_cast<int64_t>(kRowCost) * r;
     const int64_t lo = r == 0 ? -1 : static_cast<int64_t>(ro[r - 1]) + static_cast<int64_t>(kRowCost) * (r - 1);
     // chunk boundaries c * K in (lo, hi]
-    int64_t c0 = lo < 0 ? 0 : lo / kChunkCost + 1;
-    const int64_t c1 = hi / kChunkCost;
+    int64_t c0 = lo < 0 ? 0 : lo / cost + 1;
+    const int64_t c1 = hi / cost;
     for (int64_t c = c0; c <= c1 && c < nchunks; ++c) chunks[c] = r;
     if (r == rows) chunks[nchunks] = rows;
 }
@@ -217,6 +218,27 @@ int schedule(const CsrPattern32 &p, cudaStream_t s, const unsigned char *breaks,
 }
 } // namespace
 
+namespace {
+// The work of one warp-tile or chunk: `most` on a matrix that gives every SM
+// kUnitsPerSM of them, less on a smaller one, so that it reaches all SMs with
+// a short chain per warp. A x / A'y, float64, best variant, with units of 768 /
+// 1,024 and with these: 40,000 nonzeros 8.5 / 6.6 -> 6.4 / 6.1 us (the untuned
+// variant 0: 14.8 / 10.5 -> 6.5 / 6.5), 600,000 14.7 / 10.5 -> 8.4 / 8.4, 1.7
+// million 16.6 / 13.5 -> 13.7 / 13.1, 6 million 39.3 / 39.9 -> 35.5 / 35.2; 21
+// million are past the line. With 64 units per SM the 5-million power-law
+// transpose, whose chunks then match the resident warps one to one, loses 6%;
+// units capped at 512 lose 4% on the 21-million one.
+constexpr int kUnitsPerSM = 128;
+constexpr int kLeastUnit = 64;
+int work_unit(int64_t total, int most) {
+    int dev = 0, sms = 0;
+    VK_CUDA(cudaGetDevice(&dev));
+    VK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int64_t share = total / (static_cast<int64_t>(sms) * kUnitsPerSM);
+    return static_cast<int>(std::min<int64_t>(most, std::max<int64_t>(kLeastUnit, share)));
+}
+} // namespace
+
 void build_tiles(CsrPattern32 &p, cudaStream_t s, const unsigned char *breaks) {
     const int rows = p.rows;
     if (breaks) {
@@ -229,16 +251,18 @@ void build_tiles(CsrPattern32 &p, cudaStream_t s, const unsigned char *breaks) {
             if (h[r]) f = mix_fingerprint(f, r);
         p.fp = mix_fingerprint(p.fp, f);
     }
-    p.ntiles = schedule(p, s, breaks, kChunk, kShortMax, kTileRows, p.tiles, p.tile_k);
-    p.nstiles = schedule(p, s, nullptr, kStageWindow, kStageShort, kStageRows, p.stiles, p.stile_k);
+    const int window = work_unit(p.nnz, kChunk);
+    p.ntiles = schedule(p, s, breaks, window, kShortMax, kTileRows, p.tiles, p.tile_k);
+    p.nstiles = schedule(p, s, nullptr, std::min(window, kStageWindow), kStageShort, kStageRows, p.stiles, p.stile_k);
     // cost-balanced row ranges for the hybrid kernel
     int nnz_total = 0;
     VK_CUDA(cudaMemcpyAsync(&nnz_total, p.ro.get() + rows, sizeof(int), cudaMemcpyDeviceToHost, s));
     VK_CUDA(cudaStreamSynchronize(s));
     const int64_t cost = static_cast<int64_t>(nnz_total) + static_cast<int64_t>(kRowCost) * rows;
-    p.nchunks = rows > 0 ? static_cast<int>((cost - 1) / kChunkCost + 1) : 0;
+    const int unit = work_unit(cost, kChunkCost);
+    p.nchunks = rows > 0 ? static_cast<int>((cost - 1) / unit + 1) : 0;
     p.chunks.reset(p.nchunks + 1);
-    chunk_rows_kernel<<<ceil_div(rows + 1, 256), 256, 0, s>>>(p.ro.get(), rows, p.nchunks, p.chunks.get());
+    chunk_rows_kernel<<<ceil_div(rows + 1, 256), 256, 0, s>>>(p.ro.get(), rows, unit, p.nchunks, p.chunks.get());
     VK_LAUNCH_CHECK();
     VK_CUDA(cudaStreamSynchronize(s));
 }

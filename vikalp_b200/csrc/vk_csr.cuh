@@ -51,7 +51,7 @@ namespace vk {
 
 constexpr int kWarps = 4;                  // warps per CTA
 constexpr int kTileThreads = kWarps * 32;  // threads per CTA
-constexpr int kChunk = 768;                // nonzero window that groups short rows
+constexpr int kChunk = 768;                // nonzero window that groups short rows (less on small matrices: build_tiles)
 constexpr int kShortMax = 256;             // longer rows get a tile of their own
 constexpr int kCap = kChunk + kShortMax;   // max nonzeros of a multi-row tile
 constexpr int kTileRows = 64;              // max rows per warp-tile
@@ -537,8 +537,8 @@ __global__ void __launch_bounds__(kTileThreads, MINB)
 // so the epilogue's loads and stores are coalesced across the group. With
 // LATE the epilogue's inputs are loaded after the sums (other warps hide that
 // latency at full occupancy) rather than held in registers across the gathers.
-// Work: cost-balanced row ranges (chunks, about kChunkCost nonzeros-plus-4-
-// per-row each) round robin over the persistent grid, or the tile schedule's
+// Work: cost-balanced row ranges (chunks, kChunkCost nonzeros-plus-4-per-row
+// each, fewer on small matrices) round robin over the persistent grid, or the tile schedule's
 // tiles when the epilogue reduces per tile or skips tiles.
 constexpr int kChunkCost = 1024;
 constexpr int kRowCost = 4;
