@@ -82,3 +82,20 @@ def test_several_launches_and_repeated_solves():
         for k in ("x", "y"):
             assert np.max(np.abs(r[k] - want[k])) <= 1e-8 * (1.0 + np.abs(want[k]).max()), k
     assert np.array_equal(runs[0]["x"], runs[1]["x"]) and np.array_equal(runs[0]["y"], runs[1]["y"])
+
+
+@pytest.mark.parametrize("name", [k for k in MODELS if k != "qp"])
+@pytest.mark.parametrize("iterations", [1, 51, 52, 157, 1030])
+def test_reference_scheme_matches_oracle(oracle, name, iterations):
+    # FAST order: the oracle's iterates to 1e-9 through the step rule's
+    # iterations (51, 101, ...) and a second launch (over 1,024)
+    inst = MODELS[name]()
+    tol = dict(primal_tolerance=0.0, dual_tolerance=0.0)
+    want = oracle.pdhg_solve(inst, iteration_limit=iterations, **tol)
+    got = vk.solve(inst, algorithm="reference", iteration_limit=iterations, **tol)
+    if want["iterations"] == iterations:
+        assert got["iterations"] == iterations
+    else:  # one row and column: the metric reaches exactly 0, at an iteration that rounding decides
+        assert name == "one_by_one" and got["last_metric"] == 0.0
+    for k in ("x", "y"):
+        assert np.max(np.abs(got[k] - want[k]), initial=0.0) <= 1e-9 * (1.0 + np.abs(want[k]).max()), k

@@ -48,7 +48,6 @@ namespace {
 
 constexpr int kRuizPasses = 10;
 constexpr int kPowerMax = 200;
-constexpr int kRsIterations = 1024; // iterations in one launch of the resident kernel
 constexpr int64_t kTunePassesMinNnz = 2000000; // per-pass variant tuning from this many nonzeros
 
 // ---- scaling (FP64, original values) -----------------------------------------
@@ -402,14 +401,6 @@ struct HalState {
     DevBuf<T> q, qx;                        // QP: Q^ = D Q D values, Q^ x
 };
 
-// The resident launch of one precision, when the model fits (plan_resident).
-struct Resident {
-    bool on = false, small = false; // small: 16-bit indices
-    int grid = 0, threads = 0;
-    size_t smem = 0;
-    int cap_a = 0, cap_t = 0, cap_q = 0, rows = 0, cols = 0;
-};
-
 class HalpernEngine final : public Engine {
 public:
     HalpernEngine(const DeviceModel &dm, const vk_options &o, cudaStream_t s) : dm_(dm), o_(o), s_(s) {
@@ -547,7 +538,7 @@ public:
         bool confirmed = false; // mixed: the float32 answer passed the float64 evaluation
         if (mixed_) {
             copy_state<float, double>(s64_, s32_);
-            if (!rs32_.on && !g32_) g32_ = capture(s32_);
+            if (!rs32_ && !g32_) g32_ = capture(s32_);
             // float32 phase. When its own (float32) KKT evaluation reaches the
             // tolerance, the point is evaluated again in float64 with no
             // float64 iteration: accepted there, the solve ends; otherwise the
@@ -627,7 +618,7 @@ public:
             }
         }
         if (!timed_out && !confirmed) {
-            if (!rs64_.on && !g64_) g64_ = capture(s64_);
+            if (!rs64_ && !g64_) g64_ = capture(s64_);
             for (;;) {
                 if (over_time(started)) {
                     timed_out = true;
@@ -702,10 +693,10 @@ private:
     // kernel: it stops by itself; the float32 phase's plateau rule wants every
     // check, as does the trace), and the control block back on the host.
     template <class T>
-    void advance(HalState<T> &st, const Resident &r, cudaGraphExec_t g) {
-        if (r.on) {
+    void advance(HalState<T> &st, bool resident, cudaGraphExec_t g) {
+        if (resident) {
             const bool every = sizeof(T) == 4 || o_.verbose >= 2;
-            launch_resident(st, r, every ? 1 : std::max(1, kRsIterations / chunk_));
+            launch_resident(st, every ? 1 : std::max(1, kRsIterations / chunk_));
             launches_ += 1;
         } else {
             VK_CUDA(cudaGraphLaunch(g, s_));
@@ -722,65 +713,35 @@ private:
     }
 
     // A model whose matrices fit the GPU's shared memory iterates there
-    // (vk_resident.cuh). A pinned kernel variant keeps the passes.
+    // (vk_resident.cuh): 11.0 us an iteration against 23.7 for the passes at
+    // 600,000 nonzeros, 16.1 against 37.5 at 720,000 (float64; past about
+    // 800,000 they no longer fit), 17.5 against 26.4 at 940,000 (float32).
     void plan_resident() {
-        if (dm_.m == 0 || dm_.nnz == 0 || forced_variant() >= 0) return;
-        const int64_t nnz = 2 * dm_.nnz + (dm_.qp ? dm_.q_nnz : 0);
-        if (nnz * static_cast<int64_t>(sizeof(float) + 2) > static_cast<int64_t>(kRsMaxGrid) * kRsSmem) return;
-        const int m = dm_.m, n = dm_.n;
-        std::vector<int> ro(m + 1), rot(n + 1), roq(dm_.qp ? n + 1 : 0);
-        const auto get = [&](std::vector<int> &h, const DevBuf<int> &d) {
-            if (!h.empty())
-                VK_CUDA(cudaMemcpyAsync(h.data(), d.get(), h.size() * sizeof(int), cudaMemcpyDeviceToHost, s_));
-        };
-        get(ro, dm_.a.ro);
-        get(rot, dm_.at.ro);
-        get(roq, dm_.q.ro);
-        VK_CUDA(cudaStreamSynchronize(s_));
-        Resident r;
-        r.grid = rs_grid(dm_.nnz);
-        r.threads = rs_threads(dm_.nnz, r.grid);
-        r.small = m <= 65536 && n <= 65536;
-        // columns are split by their nonzeros in A and Q together
-        std::vector<int> both(rot);
-        for (size_t j = 0; j < roq.size(); ++j) both[j] += roq[j];
-        const RsPart pa = rs_partition(ro, m, r.grid), pt = rs_partition(both, n, r.grid);
-        r.rows = pa.rows;
-        r.cols = pt.rows;
-        r.cap_a = static_cast<int>(pa.nnz);
-        for (int b = 0; b < r.grid; ++b) {
-            r.cap_t = std::max(r.cap_t, rot[pt.at[b + 1]] - rot[pt.at[b]]);
-            if (dm_.qp) r.cap_q = std::max(r.cap_q, roq[pt.at[b + 1]] - roq[pt.at[b]]);
-        }
-        rs64_ = rs32_ = r;
-        plan_one<double>(rs64_);
-        if (mixed_) plan_one<float>(rs32_);
-        if (!rs64_.on && !rs32_.on) return;
-        part_a_.reset(pa.at.size());
-        part_t_.reset(pt.at.size());
-        counter_.reset(1);
+        if (!rs_plan(dm_.a, dm_.at, dm_.qp ? &dm_.q : nullptr, plan_, s_)) return;
+        fits_resident<double>(rs64_);
+        if (mixed_) fits_resident<float>(rs32_);
         partials_.reset(static_cast<size_t>(kRsMaxGrid) * kCheckSums);
-        VK_CUDA(cudaMemcpyAsync(part_a_.get(), pa.at.data(), part_a_.bytes(), cudaMemcpyHostToDevice, s_));
-        VK_CUDA(cudaMemcpyAsync(part_t_.get(), pt.at.data(), part_t_.bytes(), cudaMemcpyHostToDevice, s_));
-        VK_CUDA(cudaStreamSynchronize(s_));
     }
     template <class T>
-    void plan_one(Resident &r) {
-        with_kernel<T>(r, [&](auto kernel, auto index) {
-            r.smem = RsHalLayout<T, decltype(index)>(r.cap_a, r.cap_t, r.cap_q, r.rows, r.cols, dm_.qp).bytes;
-            r.on = rs_fits(kernel, r.grid, r.threads, r.smem);
+    void fits_resident(bool &on) {
+        with_kernel<T>([&](auto kernel, auto index) {
+            on = rs_fits(kernel, plan_.grid, plan_.threads, layout<T>(index));
         });
+    }
+    template <class T, class I>
+    size_t layout(I) const {
+        return RsHalLayout<T, I>(plan_.cap_a, plan_.cap_t, plan_.cap_q, plan_.rows, plan_.cols, dm_.qp).bytes;
     }
     // f(kernel, a value of its index type)
     template <class T, class F>
-    void with_kernel(const Resident &r, F &&f) {
+    void with_kernel(F &&f) {
         if (dm_.qp)
-            r.small ? f(rs_halpern_kernel<T, uint16_t, true>, uint16_t()) : f(rs_halpern_kernel<T, int, true>, int());
+            plan_.small ? f(rs_halpern_kernel<T, uint16_t, true>, uint16_t()) : f(rs_halpern_kernel<T, int, true>, int());
         else
-            r.small ? f(rs_halpern_kernel<T, uint16_t, false>, uint16_t()) : f(rs_halpern_kernel<T, int, false>, int());
+            plan_.small ? f(rs_halpern_kernel<T, uint16_t, false>, uint16_t()) : f(rs_halpern_kernel<T, int, false>, int());
     }
     template <class T>
-    void launch_resident(HalState<T> &st, const Resident &r, int chunks) {
+    void launch_resident(HalState<T> &st, int chunks) {
         RsHalArgs<T> a{};
         a.ro_a = dm_.a.ro.get();
         a.ci_a = dm_.a.ci.get();
@@ -791,13 +752,13 @@ private:
         a.va = st.ka.get();
         a.vt = st.kat.get();
         a.vq = st.q.get();
-        a.part_a = part_a_.get();
-        a.part_t = part_t_.get();
-        a.cap_a = r.cap_a;
-        a.cap_t = r.cap_t;
-        a.cap_q = r.cap_q;
-        a.rows = r.rows;
-        a.cols = r.cols;
+        a.part_a = plan_.part_a.get();
+        a.part_t = plan_.part_t.get();
+        a.cap_a = plan_.cap_a;
+        a.cap_t = plan_.cap_t;
+        a.cap_q = plan_.cap_q;
+        a.rows = plan_.rows;
+        a.cols = plan_.cols;
         a.x = st.x.get();
         a.x0 = st.x0.get();
         a.xbar = st.xbar.get();
@@ -814,12 +775,14 @@ private:
         a.rs = st.rs.get();
         a.ctl = ctl_.get();
         a.partials = partials_.get();
-        a.counter = counter_.get();
+        a.counter = plan_.counter.get();
         a.err = device_error_flag();
         a.chunk = chunk_;
         a.chunks = chunks;
-        VK_CUDA(cudaMemsetAsync(counter_.get(), 0, sizeof(unsigned), s_));
-        with_kernel<T>(r, [&](auto kernel, auto) { rs_launch(kernel, r.grid, r.threads, r.smem, s_, a); });
+        VK_CUDA(cudaMemsetAsync(plan_.counter.get(), 0, sizeof(unsigned), s_));
+        with_kernel<T>([&](auto kernel, auto index) {
+            rs_launch(kernel, plan_.grid, plan_.threads, layout<T>(index), s_, a);
+        });
     }
 
     // Ruiz (infinity norm) passes, then one Pock-Chambolle (alpha = 1) pass.
@@ -1132,9 +1095,8 @@ private:
     double knorm_ = 0.0, lq_ = 0.0, omega0_ = 1.0, bnorm_ = 0.0, cnorm_ = 0.0;
     cudaGraphExec_t g64_ = nullptr, g32_ = nullptr;
     long long graph_nodes_ = 0, launches_ = 0;
-    Resident rs64_, rs32_;
-    DevBuf<int> part_a_, part_t_;
-    DevBuf<unsigned> counter_;
+    RsPlan plan_;
+    bool rs64_ = false, rs32_ = false; // the model is resident in float64 / float32
     DevBuf<double> partials_;
     bool tuned_ = false;
     int col_var_[2] = {-1, -1}, row_var_[2] = {-1, -1}; // tuned pass variants [float64, float32]

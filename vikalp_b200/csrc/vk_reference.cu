@@ -30,6 +30,7 @@
 // Chunks of iterations are captured in a CUDA graph; the host only polls a
 // done flag between chunks.
 #include "vk_engine.cuh"
+#include "vk_reference_resident.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -169,11 +170,6 @@ struct RefRowEpi : EpiBase<double> {
     }
 };
 
-// True when the control step of iteration k (which judges the metric of
-// iteration k-1) may change tau / sigma or set the restart flag: pdhg.cpp:133,
-// every 50 iterations after the first.
-__device__ __forceinline__ bool ref_policy_iter(long long k) { return k >= 51 && (k - 1) % 50 == 0; }
-
 // FAST column pass: the stationarity norm of iteration k-1 as RefColEpi, and
 // the primal step of iteration k (ref_primal_kernel's arithmetic) in the same
 // epilogue unless the control step may still change tau; then K'y goes to aty
@@ -200,14 +196,8 @@ struct RefColFastEpi : EpiBase<double> {
             return;
         }
         const double tau = __ldg(&ctl->tau);
-        double v;
-        if (QP) {
-            v = __dadd_rn(__dmul_rn(-tau, g), p.x);
-        } else {
-            const double t = __dadd_rn(__dmul_rn(-tau, p.c), p.x);
-            v = __dadd_rn(__dmul_rn(-tau, s[0]), t);
-        }
-        xn[j] = clampbox(v, p.l, p.u);
+        xn[j] = QP ? clampbox(__dadd_rn(__dmul_rn(-tau, g), p.x), p.l, p.u)
+                   : ref_primal(tau, s[0], p.x, p.c, p.l, p.u);
     }
     __device__ void finish(double (&red)[1], double *scratch, int) const {
         const double v = block_max_nonneg(red[0], scratch);
@@ -255,42 +245,11 @@ struct StoreEpi : EpiRow<double, StoreEpi> {
     __device__ void row(int i, const double (&s)[1], double (&)[1]) const { out[i] = s[0]; }
 };
 
-// The metric of iteration k-1 and the step / restart / stop rules
-// (pdhg.cpp:133-150). One thread.
+// The control step (ref_decide). One thread.
 __global__ void ref_control_kernel(RefCtl *ctl) {
     RefCtl c = *ctl;
     if (c.done) return;
-    c.restart = 0; // consumed by the previous primal step (pdhg.cpp:98-100)
-    if (c.iter >= 1) {
-        const long long it = c.iter - 1;
-        const double metric = smax(c.rp, c.rd);
-        c.last_metric = metric;
-        if (it > 0 && it % 50 == 0) {
-            if (metric > c.previous * 1.25) {
-                c.tau *= 0.5;
-                c.sigma *= 0.5;
-                c.restart = 1;
-                c.restarts += 1;
-            } else if (metric < c.previous * 0.1) {
-                c.tau = smin(c.tau * 1.05, c.max_step);
-                c.sigma = c.tau;
-            }
-            c.previous = metric;
-        } else if (it == 0) {
-            c.previous = metric;
-        }
-        if (metric <= c.tol) {
-            c.done = 1;
-            c.status = VK_STATUS_OPTIMAL;
-        }
-    }
-    if (!c.done && c.iter >= c.limit) {
-        c.done = 1;
-        c.status = VK_STATUS_ITERATION_LIMIT;
-    }
-    c.inv_sigma = 1.0 / c.sigma;
-    c.rp = 0.0;
-    c.rd = 0.0;
+    ref_decide(c);
     *ctl = c;
 }
 
@@ -392,7 +351,8 @@ public:
         const int64_t work = dm.nnz + dm.m + dm.n;
         graph_iters_ = work < (1 << 20) ? 128 : (work < (1 << 24) ? 32 : 8);
         if (!exact_) graph_iters_ = work < (1 << 20) ? 150 : 50;
-        tune_passes();
+        plan_resident();
+        if (!resident_) tune_passes();
     }
 
     ~ReferenceEngine() override {
@@ -431,6 +391,7 @@ public:
         const int m = dm_.m, n = dm_.n;
         prepare(nullptr, dm_.vl.get(), dm_.vu.get(), iterations, 0.0);
         const int kinds = 3;
+        if (resident_) return profile_resident(iterations, pp);
         std::vector<cudaEvent_t> ev(static_cast<size_t>(iterations) * (kinds + 1));
         for (auto &e : ev) VK_CUDA(cudaEventCreate(&e));
         for (long long k = 0; k < iterations; ++k)
@@ -439,6 +400,7 @@ public:
         check_device_error(s_);
         pp = PassProfile{};
         pp.count = kinds;
+        profile_bytes(pp);
         // names carry the kernel variant each pass ran (the tuner's pick)
         const auto tag = [&](int v) { return exact_ ? std::string(", sequential") : ", variant " + std::to_string(v); };
         prof_names_[0] = "column pass (K'y, primal step)" + tag(col_view().variant);
@@ -446,14 +408,6 @@ public:
         prof_names_[2] = (dm_.qp ? std::string("Q pass + row pass") : std::string("row pass (K x, dual step)")) +
                          tag(row_view().variant);
         for (int q = 0; q < kinds; ++q) pp.name[q] = prof_names_[q].c_str();
-        const double s = 8.0; // float64 values and vectors
-        const double nnz = static_cast<double>(dm_.nnz);
-        // Algorithmic bytes: values + int32 indices, int32 offsets, the
-        // gathered vector once, the per-row / per-column vectors of the
-        // epilogue (see the epilogues above).
-        pp.bytes[0] = nnz * (s + 4) + 4.0 * (n + 1) + s * m + s * n * (dm_.qp ? 6 : 5);
-        pp.bytes[1] = 0.0;
-        pp.bytes[2] = nnz * (s + 4) + 4.0 * (m + 1) + s * n + s * m * (exact_ ? 4 : 6) + (exact_ ? s * n : 0.0);
         for (long long k = 0; k < iterations; ++k) {
             for (int q = 0; q < kinds; ++q) {
                 float ms = 0.f;
@@ -467,11 +421,57 @@ public:
         return true;
     }
 
+    void profile_bytes(PassProfile &pp) const {
+        const int m = dm_.m, n = dm_.n;
+        const double s = 8.0; // float64 values and vectors
+        const double nnz = static_cast<double>(dm_.nnz);
+        // Algorithmic bytes: values + int32 indices, int32 offsets, the
+        // gathered vector once, the per-row / per-column vectors of the
+        // epilogue (see the epilogues above).
+        pp.bytes[0] = nnz * (s + 4) + 4.0 * (n + 1) + s * m + s * n * (dm_.qp ? 6 : 5);
+        pp.bytes[1] = 0.0;
+        pp.bytes[2] = nnz * (s + 4) + 4.0 * (m + 1) + s * n + s * m * (exact_ ? 4 : 6) + (exact_ ? s * n : 0.0);
+    }
+
+    // A resident model: the iterations' device time, divided by the cycles that
+    // CTA 0 counted in the three parts of an iteration.
+    bool profile_resident(long long iterations, PassProfile &pp) {
+        DevBuf<long long> cycles(3);
+        VK_CUDA(cudaMemsetAsync(cycles.get(), 0, cycles.bytes(), s_));
+        cudaEvent_t e0, e1;
+        VK_CUDA(cudaEventCreate(&e0));
+        VK_CUDA(cudaEventCreate(&e1));
+        VK_CUDA(cudaEventRecord(e0, s_));
+        for (long long k = 0; k < iterations; k += kRsIterations) launch_resident(cycles.get());
+        VK_CUDA(cudaEventRecord(e1, s_));
+        long long h[3];
+        VK_CUDA(cudaMemcpyAsync(h, cycles.get(), sizeof(h), cudaMemcpyDeviceToHost, s_));
+        VK_CUDA(cudaStreamSynchronize(s_));
+        check_device_error(s_);
+        float ms = 0.f;
+        VK_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+        pp = PassProfile{};
+        pp.count = 3;
+        profile_bytes(pp);
+        prof_names_[0] = "column pass (K'y, primal step), resident";
+        prof_names_[1] = "control";
+        prof_names_[2] = "row pass (K x, dual step), resident";
+        const double all = static_cast<double>(std::max<long long>(1, h[0] + h[1] + h[2]));
+        for (int q = 0; q < 3; ++q) {
+            pp.name[q] = prof_names_[q].c_str();
+            pp.ms[q] = ms * static_cast<double>(std::max<long long>(1, h[q])) / all;
+            pp.launches[q] = iterations;
+        }
+        return true;
+    }
+
     void run(const double *d_warm, const double *d_lo, const double *d_hi, double *d_xo, double *d_yo,
              RunInfo &info, std::chrono::steady_clock::time_point started) override {
         const int m = dm_.m, n = dm_.n;
         prepare(d_warm, d_lo, d_hi, o_.iteration_limit, smax(o_.primal_tolerance, o_.dual_tolerance));
-        if (!graph_exec_) capture();
+        if (!resident_ && !graph_exec_) capture();
         cudaEvent_t e0, e1;
         VK_CUDA(cudaEventCreate(&e0));
         VK_CUDA(cudaEventCreate(&e1));
@@ -482,8 +482,13 @@ public:
                 timed_out = true;
                 break;
             }
-            VK_CUDA(cudaGraphLaunch(graph_exec_, s_));
-            info.kernel_launches += graph_nodes_;
+            if (resident_) {
+                launch_resident();
+                info.kernel_launches += 1;
+            } else {
+                VK_CUDA(cudaGraphLaunch(graph_exec_, s_));
+                info.kernel_launches += graph_nodes_;
+            }
             VK_CUDA(cudaMemcpyAsync(hctl_.get(), ctl_.get(), sizeof(RefCtl), cudaMemcpyDeviceToHost, s_));
             VK_CUDA(cudaStreamSynchronize(s_));
             check_device_error(s_);
@@ -502,7 +507,7 @@ public:
         info.last_metric = h.last_metric;
         info.status = timed_out && !h.done ? VK_STATUS_TIME_LIMIT : h.status;
         info.iterate_seconds = ms * 1e-3;
-        const double *xf = x_[h.iter % 2].get();
+        const double *xf = resident_ ? x_[0].get() : x_[h.iter % 2].get();
         unscale_kernel<<<grid1d(n), 256, 0, s_>>>(xf, cs_.get(), n, d_xo);
         if (m > 0) unscale_kernel<<<grid1d(m), 256, 0, s_>>>(y_.get(), rs_.get(), m, d_yo);
         VK_LAUNCH_CHECK();
@@ -524,6 +529,56 @@ private:
         e.ctl = ctl;
         e.out = qx_.get();
         tiles(view(dm_.q, kq_.get()), Gathers<double, 1>{{x}}, e);
+    }
+
+    // A FAST-order LP whose matrices fit the GPU's shared memory iterates there
+    // (vk_resident.cuh); pinned variants keep the passes.
+    void plan_resident() {
+        const char *pinned = std::getenv("VIKALP_B200_PASS_VARIANTS");
+        if (exact_ || dm_.qp || (pinned && *pinned) || !rs_plan(dm_.a, dm_.at, nullptr, plan_, s_)) return;
+        resident_ = plan_.small ? rs_fits(rs_reference_kernel<uint16_t>, plan_.grid, plan_.threads, layout<uint16_t>())
+                                : rs_fits(rs_reference_kernel<int>, plan_.grid, plan_.threads, layout<int>());
+        norms_.reset(8);
+    }
+    template <class I>
+    size_t layout() const {
+        return RsRefLayout<I>(plan_.cap_a, plan_.cap_t, plan_.rows, plan_.cols).bytes;
+    }
+    void launch_resident(long long *cycles = nullptr) {
+        RsRefArgs a{};
+        a.cycles = cycles;
+        a.ro_a = dm_.a.ro.get();
+        a.ci_a = dm_.a.ci.get();
+        a.ro_t = dm_.at.ro.get();
+        a.ci_t = dm_.at.ci.get();
+        a.va = ka_.get();
+        a.vt = kat_.get();
+        a.part_a = plan_.part_a.get();
+        a.part_t = plan_.part_t.get();
+        a.cap_a = plan_.cap_a;
+        a.cap_t = plan_.cap_t;
+        a.rows = plan_.rows;
+        a.cols = plan_.cols;
+        a.x = x_[0].get();
+        a.xn = x_[1].get();
+        a.y = y_.get();
+        a.kx = kx_.get();
+        a.c = sc_.get();
+        a.l = sl_.get();
+        a.u = su_.get();
+        a.rl = srl_.get();
+        a.ru = sru_.get();
+        a.ctl = ctl_.get();
+        a.norms = norms_.get();
+        a.counter = plan_.counter.get();
+        a.err = device_error_flag();
+        a.iterations = kRsIterations;
+        VK_CUDA(cudaMemsetAsync(plan_.counter.get(), 0, sizeof(unsigned), s_));
+        VK_CUDA(cudaMemsetAsync(norms_.get(), 0, norms_.bytes(), s_));
+        if (plan_.small)
+            rs_launch(rs_reference_kernel<uint16_t>, plan_.grid, plan_.threads, layout<uint16_t>(), s_, a);
+        else
+            rs_launch(rs_reference_kernel<int>, plan_.grid, plan_.threads, layout<int>(), s_, a);
     }
 
     void iteration(int k) { iteration_parts(k, nullptr); }
@@ -744,6 +799,9 @@ private:
     int col_variant_ = -1, row_variant_ = -1; // tuned kernel variants of the fused passes (-1: the pattern's)
     long long graph_nodes_ = 0;
     cudaGraphExec_t graph_exec_ = nullptr;
+    RsPlan plan_;
+    bool resident_ = false;
+    DevBuf<double> norms_;
 };
 
 __global__ void bump_iter_kernel(RefCtl *ctl) {

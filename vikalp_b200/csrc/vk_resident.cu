@@ -3,14 +3,15 @@
 
 namespace vk {
 
-RsPart rs_partition(const std::vector<int> &ro, int rows, int ctas) {
-    RsPart p;
-    p.at.assign(static_cast<size_t>(ctas) + 1, rows);
-    p.at[0] = 0;
+namespace {
+// Boundaries of `rows` rows over `ctas` shares of about equal cost.
+std::vector<int> partition(const std::vector<int> &ro, int rows, int ctas) {
+    std::vector<int> at(static_cast<size_t>(ctas) + 1, rows);
+    at[0] = 0;
     const auto cost = [&](int r) { return static_cast<int64_t>(ro[r]) + static_cast<int64_t>(kRsRowCost) * r; };
     const int64_t total = cost(rows);
     for (int b = 1; b < ctas; ++b) {
-        int lo = p.at[b - 1], hi = rows; // the first row at or past the share's start
+        int lo = at[b - 1], hi = rows; // the first row at or past the share's start
         while (lo < hi) {
             const int mid = (lo + hi) / 2;
             if (cost(mid) * ctas < total * b)
@@ -18,13 +19,53 @@ RsPart rs_partition(const std::vector<int> &ro, int rows, int ctas) {
             else
                 hi = mid;
         }
-        p.at[b] = lo;
+        at[b] = lo;
     }
-    for (int b = 0; b < ctas; ++b) {
-        p.rows = std::max(p.rows, p.at[b + 1] - p.at[b]);
-        p.nnz = std::max<int64_t>(p.nnz, ro[p.at[b + 1]] - ro[p.at[b]]);
-    }
-    return p;
+    return at;
+}
+
+int largest_share(const std::vector<int> &ro, const std::vector<int> &at) {
+    int most = 0;
+    for (size_t b = 0; b + 1 < at.size(); ++b) most = std::max(most, ro[at[b + 1]] - ro[at[b]]);
+    return most;
+}
+
+int most_rows(const std::vector<int> &at) {
+    int most = 0;
+    for (size_t b = 0; b + 1 < at.size(); ++b) most = std::max(most, at[b + 1] - at[b]);
+    return most;
+}
+} // namespace
+
+bool rs_plan(const CsrPattern32 &a, const CsrPattern32 &at, const CsrPattern32 *q, RsPlan &plan, cudaStream_t s) {
+    if (a.rows == 0 || a.nnz == 0 || forced_variant() >= 0) return false;
+    const int64_t stored = 2 * a.nnz + (q ? q->nnz : 0);
+    if (stored * static_cast<int64_t>(sizeof(float) + 2) > static_cast<int64_t>(kRsMaxGrid) * kRsSmem) return false;
+    const int m = a.rows, n = a.cols;
+    std::vector<int> ro(m + 1), rot(n + 1), roq(q ? n + 1 : 0);
+    VK_CUDA(cudaMemcpyAsync(ro.data(), a.ro.get(), ro.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
+    VK_CUDA(cudaMemcpyAsync(rot.data(), at.ro.get(), rot.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
+    if (q) VK_CUDA(cudaMemcpyAsync(roq.data(), q->ro.get(), roq.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
+    VK_CUDA(cudaStreamSynchronize(s));
+    plan.grid = rs_grid(a.nnz);
+    plan.threads = rs_threads(a.nnz, plan.grid);
+    plan.small = m <= 65536 && n <= 65536;
+    // columns are split by their nonzeros in A and Q together
+    std::vector<int> both(rot);
+    for (size_t j = 0; j < roq.size(); ++j) both[j] += roq[j];
+    const std::vector<int> pa = partition(ro, m, plan.grid), pt = partition(both, n, plan.grid);
+    plan.rows = most_rows(pa);
+    plan.cols = most_rows(pt);
+    plan.cap_a = largest_share(ro, pa);
+    plan.cap_t = largest_share(rot, pt);
+    plan.cap_q = q ? largest_share(roq, pt) : 0;
+    plan.part_a.reset(pa.size());
+    plan.part_t.reset(pt.size());
+    plan.counter.reset(1);
+    VK_CUDA(cudaMemcpyAsync(plan.part_a.get(), pa.data(), plan.part_a.bytes(), cudaMemcpyHostToDevice, s));
+    VK_CUDA(cudaMemcpyAsync(plan.part_t.get(), pt.data(), plan.part_t.bytes(), cudaMemcpyHostToDevice, s));
+    VK_CUDA(cudaStreamSynchronize(s)); // the boundaries live on this stack frame
+    return true;
 }
 
 int rs_grid(int64_t nnz) {

@@ -30,14 +30,8 @@ constexpr int kRsRowCost = 4;       // partition: a row costs this many nonzeros
 constexpr int kRsGather = 4;        // gathers in flight per thread
 constexpr int kRsWarpRow = 32;      // a row of more than this many products per lane goes to a whole warp
 constexpr int kRsMaxGrid = 160;
+constexpr int kRsIterations = 1024; // iterations in one launch, about
 constexpr unsigned kRsPolls = 1u << 25; // over ten seconds
-
-// Rows [part[b], part[b+1]) of a matrix belong to CTA b; the largest shares.
-struct RsPart {
-    int rows = 0;
-    int64_t nnz = 0;
-    std::vector<int> at;
-};
 
 // ---- device side ----------------------------------------------------------------
 
@@ -136,6 +130,23 @@ struct RsBarrier {
     // False when another CTA never came: the caller returns.
     __device__ __forceinline__ bool sync() {
         __syncthreads();
+        return arrive_and_wait();
+    }
+    // The same, and *slot becomes the largest of itself and every thread's v
+    // (non-negative; NaN ignored). `warps`: 32 doubles of shared memory.
+    __device__ __forceinline__ bool sync_max(double v, double *warps, double *slot) {
+        v = warp_max_nonneg(v);
+        if ((threadIdx.x & 31) == 0) warps[threadIdx.x >> 5] = v;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (unsigned w = 1; w < blockDim.x / 32; ++w) v = smax(v, warps[w]);
+            atomic_max_nonneg(slot, v);
+        }
+        return arrive_and_wait();
+    }
+
+private:
+    __device__ __forceinline__ bool arrive_and_wait() {
         target += gridDim.x;
         bool ok = true;
         if (threadIdx.x == 0) {
@@ -171,8 +182,18 @@ __device__ __forceinline__ bool rs_sum(double (&v)[NR], double *partials, double
 
 // ---- host side (vk_resident.cu) ------------------------------------------------------
 
-// Splits `rows` rows over `ctas` shares of about equal cost.
-RsPart rs_partition(const std::vector<int> &ro, int rows, int ctas);
+// The launch of a model: its shape, the largest shares, the shares' boundaries.
+struct RsPlan {
+    bool small = false; // 16-bit indices
+    int grid = 0, threads = 0;
+    int cap_a = 0, cap_t = 0, cap_q = 0, rows = 0, cols = 0;
+    DevBuf<int> part_a, part_t;
+    DevBuf<unsigned> counter; // of the grid barrier
+};
+
+// Fills `plan` for A, its transpose and (or null) Q; false when the matrices
+// can not fit in any precision, or a kernel variant is pinned.
+bool rs_plan(const CsrPattern32 &a, const CsrPattern32 &at, const CsrPattern32 *q, RsPlan &plan, cudaStream_t s);
 
 // CTAs (at most one per SM) and threads for `nnz` nonzeros. Timed per
 // iteration (float64 Halpern, 37 / 74 / 148 CTAs x 256 / 512 / 768 / 1024
