@@ -105,3 +105,40 @@ def test_autograd_function(lps, highs):
     assert rel(b.grad.numpy(), want["b"]) <= GRAD_TOL
     assert rel(a.grad.numpy(), want["A"]) <= GRAD_TOL
     assert torch.all(c.grad == 0)
+
+
+def _planted(m, n, free, per_col, seed):
+    """A model with a known optimum: every row active, `free` columns inside
+    their bounds (fewer than rows, so the adjoint system is consistent)."""
+    rng = np.random.default_rng(seed)
+    inst = synthetic.lp_uniform(m, n, per_col, seed=seed)
+    x = np.where(np.arange(n) < free, rng.uniform(1, 9, n), 0.0)
+    ax = synthetic.csr_matvec(inst.row_offsets, inst.col_idx, inst.values, x)
+    inst.row_lower, inst.row_upper = np.full(m, -np.inf), ax
+    return inst, x, rng.uniform(0, 1, m)
+
+
+def test_instances_that_fit_one_sm_and_one_that_does_not():
+    # the last instance's kept nonzeros (2,000 free columns x 8) exceed one
+    # SM's shared memory; the others take one CTA each: a single row, no free
+    # column, one free column, a zero gradient, an odd size. Against the dense
+    # minimum-norm solution; 1e-8 as at the oracle's point (LSQR to 1e-12,
+    # condition numbers below 1e3).
+    shapes = [(1, 3, 1, 1), (40, 60, 0, 3), (40, 60, 1, 3), (333, 701, 200, 7), (333, 701, 200, 7), (2500, 3500, 2000, 8)]
+    models = [_planted(*s, seed=50 + k) for k, s in enumerate(shapes)]
+    rng = np.random.default_rng(9)
+    gs = [rng.standard_normal(i.n) for i, _, _ in models]
+    gs[3][:] = 0.0
+    got = vk.lp_adjoint([t[0] for t in models], [t[1] for t in models], [t[2] for t in models], gs, 0.5,
+                        solve_tolerance=1e-12)
+    for (inst, x, y), (m, n, free, _), g, r in zip(models, shapes, gs, got):
+        assert r["status"] == "Optimal" and r["rows_active"] == m and r["cols_free"] == free
+        M = inst.dense()[:, :free].T
+        keep = np.abs(M).sum(axis=1) > 0
+        w = M[keep].T @ np.linalg.solve(M[keep] @ M[keep].T, g[:free][keep]) if keep.any() else np.zeros(m)
+        want = {"b": w - 0.5 * y, "c": 0.5 * x}
+        rows = np.repeat(np.arange(m), np.diff(inst.row_offsets))
+        want["A"] = -want["b"][rows] * x[inst.col_idx]
+        for k in want:
+            if np.linalg.norm(want[k]) > 0:
+                assert rel(r[k], want[k]) <= 1e-8, (m, k, rel(r[k], want[k]))
