@@ -14,6 +14,7 @@
 // chunk of check_every iterations is one CUDA graph.
 #include "vk_blockdiag.cuh"
 #include "vk_engine.cuh"
+#include "vk_power.cuh"
 #include "vk_stage.cuh"
 
 #include <algorithm>
@@ -192,12 +193,6 @@ struct BKktColEpi : EpiBase<T> {
     }
 };
 
-template <class T>
-struct BStore : EpiRow<T, BStore<T>> {
-    T *y;
-    __device__ void row(int i, const T (&s)[1], double (&)[1]) const { y[i] = s[0]; }
-};
-
 // out[b*R + r] = sum of partials over tiles [begin[b], begin[b+1]) (fixed order).
 __global__ void segment_reduce_kernel(const double *__restrict__ partials, const int *__restrict__ begin, int count,
                                       int R, double *__restrict__ out) {
@@ -225,15 +220,6 @@ __global__ void segment_norm2_kernel(const T *__restrict__ a, const int *__restr
         s[0] += static_cast<double>(a[i]) * static_cast<double>(a[i]);
     block_sum<1>(s, scratch);
     if (threadIdx.x == 0) out[b] = s[0];
-}
-
-template <class T>
-__global__ void segment_scale_kernel(T *__restrict__ a, const int *__restrict__ inst, int n,
-                                     const double *__restrict__ nrm2) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double v = nrm2[inst[i]];
-    if (v > 0.0) a[i] = static_cast<T>(a[i] / sqrt(v));
 }
 
 __global__ void bscaled_norm_kernel(const int *__restrict__ ro, const int *__restrict__ ci,
@@ -702,42 +688,36 @@ private:
     // Per-instance power iteration (segment norms), omega_0 per instance.
     void step_sizes() {
         const int n = n_, m = m_;
-        DevBuf<double> v(n), w(m > 0 ? m : 1), z(n), nrm(B_);
+        DevBuf<double> v(n), w(m > 0 ? m : 1), nrm(B_);
         DevBuf<int> coff;
         up(coff, col_off_);
         bseed_kernel<<<grid1d(n), 256, 0, s_>>>(v.get(), cinst_.get(), coff.get(), n);
         VK_LAUNCH_CHECK();
         segment_norm2_kernel<double><<<B_, 256, 0, s_>>>(v.get(), coff.get(), B_, nrm.get());
-        segment_scale_kernel<double><<<grid1d(n), 256, 0, s_>>>(v.get(), cinst_.get(), n, nrm.get());
-        // Each instance keeps the estimate of the iteration at which its own
-        // sequence settled (the single-instance stopping rule); the shared
-        // loop runs until every instance has settled.
-        std::vector<double> est(B_, 0.0), prev(B_, 0.0), h(B_);
-        std::vector<char> settled(B_, 0);
+        // Each instance keeps the estimate of the step at which its own sequence
+        // settled (the single-instance stopping rule).
+        std::vector<double> est(B_, 0.0);
         if (nnz_ > 0 && m > 0) {
-            for (int it = 0; it < 200; ++it) {
-                BStore<double> ew;
+            DevBuf<double> sums(std::max(at_.ntiles, 1));
+            PowerState power;
+            power_start(power, B_, nrm.get(), s_);
+            power_run(power, [&] {
+                PowerEpi<false> ew;
                 ew.y = w.get();
+                ew.inv = power.inv.get();
+                ew.inst = rinst_.get();
+                ew.partials = nullptr;
                 launch_tiles<double, double, 1, false>(view(a_, s64_.ka.get()), Gathers<double, 1>{{v.get()}}, ew, s_);
-                BStore<double> ez;
-                ez.y = z.get();
+                PowerEpi<true> ez;
+                ez.y = v.get();
+                ez.inv = nullptr;
+                ez.inst = nullptr;
+                ez.partials = sums.get();
                 launch_tiles<double, double, 1, false>(view(at_, s64_.kat.get()), Gathers<double, 1>{{w.get()}}, ez, s_);
-                segment_norm2_kernel<double><<<B_, 256, 0, s_>>>(z.get(), coff.get(), B_, nrm.get());
-                VK_CUDA(cudaMemcpyAsync(h.data(), nrm.get(), B_ * 8, cudaMemcpyDeviceToHost, s_));
-                VK_CUDA(cudaStreamSynchronize(s_));
-                segment_scale_kernel<double><<<grid1d(n), 256, 0, s_>>>(z.get(), cinst_.get(), n, nrm.get());
-                std::swap(v, z);
-                bool all = true;
-                for (int b = 0; b < B_; ++b) {
-                    if (settled[b]) continue;
-                    const double e = std::sqrt(std::sqrt(h[b]));
-                    if (it > 10 && std::abs(e - prev[b]) <= 1e-6 * e) settled[b] = 1;
-                    else all = false;
-                    prev[b] = e;
-                    est[b] = e;
-                }
-                if (all) break;
-            }
+                power_control(power, sums.get(), tbeg_at_.get(), 0, true, s_);
+            }, s_);
+            VK_CUDA(cudaMemcpyAsync(est.data(), power.est.get(), B_ * sizeof(double), cudaMemcpyDeviceToHost, s_));
+            VK_CUDA(cudaStreamSynchronize(s_));
         }
         h_eta_.resize(B_);
         for (int b = 0; b < B_; ++b) h_eta_[b] = est[b] > 0.0 ? 0.99 / est[b] : 1.0;

@@ -37,6 +37,7 @@
 // (the polish). The answer is always checked in float64.
 #include "vk_engine.cuh"
 #include "vk_halpern_resident.cuh"
+#include "vk_power.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -47,7 +48,6 @@ namespace vk {
 namespace {
 
 constexpr int kRuizPasses = 10;
-constexpr int kPowerMax = 200;
 constexpr int64_t kTunePassesMinNnz = 2000000; // per-pass variant tuning from this many nonzeros
 
 // ---- scaling (FP64, original values) -----------------------------------------
@@ -119,13 +119,6 @@ __global__ void dot_kernel(const T *__restrict__ a, const T *__restrict__ b, int
     double v[1] = {s};
     block_sum<1>(v, scratch);
     if (threadIdx.x == 0) partial[blockIdx.x] = v[0];
-}
-
-template <class T>
-__global__ void scal_kernel(T *__restrict__ a, int n, const double *__restrict__ nrm2) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const double s = *nrm2 > 0.0 ? 1.0 / sqrt(*nrm2) : 1.0;
-    if (i < n) a[i] = static_cast<T>(a[i] * s);
 }
 
 // the power iteration's start vector, a hash of each column's index in the
@@ -277,12 +270,6 @@ struct QStore : EpiRow<T, QStore<T>> {
     const HalCtl *ctl;
     T *y;
     __device__ bool skip() const { return ctl->done != 0; }
-    __device__ void row(int i, const T (&s)[1], double (&)[1]) const { y[i] = s[0]; }
-};
-
-template <class T>
-struct PlainStore : EpiRow<T, PlainStore<T>> {
-    T *y;
     __device__ void row(int i, const T (&s)[1], double (&)[1]) const { y[i] = s[0]; }
 };
 
@@ -851,66 +838,51 @@ private:
     void step_size() {
         const int m = dm_.m, n = dm_.n;
         DevBuf<double> v(n), w(m > 0 ? m : 1), z(n), part(1024), nrm(1);
-        seed_kernel<<<grid1d(n), 256, 0, s_>>>(v.get(), n, dm_.reordered() ? dm_.cperm.get() : nullptr);
-        VK_LAUNCH_CHECK();
-        auto norm2 = [&](const double *a, int k) {
-            dot_kernel<double><<<std::min(1024, grid1d(k)), 256, 0, s_>>>(a, a, k, part.get());
-            reduce_partials(part.get(), std::min(1024, grid1d(k)), 1, nrm.get(), s_);
+        DevBuf<double> sums(kMaxGrid);
+        PowerState power;
+        const auto seed = [&] {
+            seed_kernel<<<grid1d(n), 256, 0, s_>>>(v.get(), n, dm_.reordered() ? dm_.cperm.get() : nullptr);
+            VK_LAUNCH_CHECK();
+            dot_kernel<double><<<std::min(1024, grid1d(n)), 256, 0, s_>>>(v.get(), v.get(), n, part.get());
+            reduce_partials(part.get(), std::min(1024, grid1d(n)), 1, nrm.get(), s_);
+            power_start(power, 1, nrm.get(), s_);
         };
-        double sigma_max = 0.0;
-        if (dm_.nnz > 0 && m > 0) {
-            norm2(v.get(), n);
-            scal_kernel<double><<<grid1d(n), 256, 0, s_>>>(v.get(), n, nrm.get());
-            double prev = 0.0;
-            for (int it = 0; it < kPowerMax; ++it) {
-                PlainStore<double> ew;
-                ew.y = w.get();
-                launch_tiles<double, double, 1, false>(view(dm_.a, s64_.ka.get()), Gathers<double, 1>{{v.get()}}, ew, s_);
-                PlainStore<double> ez;
-                ez.y = z.get();
-                launch_tiles<double, double, 1, false>(view(dm_.at, s64_.kat.get()), Gathers<double, 1>{{w.get()}}, ez,
-                                                       s_);
-                norm2(z.get(), n);
-                double h = 0.0;
-                VK_CUDA(cudaMemcpyAsync(&h, nrm.get(), sizeof(double), cudaMemcpyDeviceToHost, s_));
-                VK_CUDA(cudaStreamSynchronize(s_));
-                const double est = std::sqrt(std::sqrt(h)); // |K'K v| with |v| = 1 -> sigma_max^2
-                scal_kernel<double><<<grid1d(n), 256, 0, s_>>>(z.get(), n, nrm.get());
-                std::swap(v, z);
-                if (it > 10 && std::abs(est - prev) <= 1e-6 * est) {
-                    prev = est;
-                    break;
-                }
-                prev = est;
-            }
-            sigma_max = prev;
+        // out = M in, scaled by 1 / |v| and / or with the CTAs' sums of squares
+        const auto pass = [&](const CsrPattern32 &p, const double *val, const double *in, double *out, bool scaled,
+                              bool norm) {
+            PowerEpi<false> e;
+            e.y = out;
+            e.inv = scaled ? power.inv.get() : nullptr;
+            e.inst = nullptr;
+            e.partials = norm ? sums.get() : nullptr;
+            return launch_tiles<double, double, 1, false>(view(p, val), Gathers<double, 1>{{in}}, e, s_);
+        };
+        const auto estimate = [&] {
+            double e = 0.0;
+            VK_CUDA(cudaMemcpyAsync(&e, power.est.get(), sizeof(double), cudaMemcpyDeviceToHost, s_));
+            VK_CUDA(cudaStreamSynchronize(s_));
+            return e;
+        };
+        knorm_ = 0.0;
+        if (dm_.nnz > 0 && m > 0) { // |K'K v| at |v| = 1 -> sigma_max^2
+            seed();
+            power_run(power, [&] {
+                pass(dm_.a, s64_.ka.get(), v.get(), w.get(), true, false);
+                const int grid = pass(dm_.at, s64_.kat.get(), w.get(), v.get(), false, true);
+                power_control(power, sums.get(), nullptr, grid, true, s_);
+            }, s_);
+            knorm_ = estimate();
         }
-        knorm_ = sigma_max;
         // lambda_max(Q^) by power iteration on Q^ (PSD), same start and stopping rule
         lq_ = 0.0;
         if (dm_.qp && dm_.q_nnz > 0) {
-            seed_kernel<<<grid1d(n), 256, 0, s_>>>(v.get(), n, dm_.reordered() ? dm_.cperm.get() : nullptr);
-            norm2(v.get(), n);
-            scal_kernel<double><<<grid1d(n), 256, 0, s_>>>(v.get(), n, nrm.get());
-            double prev = 0.0;
-            for (int it = 0; it < kPowerMax; ++it) {
-                PlainStore<double> ez;
-                ez.y = z.get();
-                launch_tiles<double, double, 1, false>(view(dm_.q, s64_.q.get()), Gathers<double, 1>{{v.get()}}, ez, s_);
-                norm2(z.get(), n);
-                double h = 0.0;
-                VK_CUDA(cudaMemcpyAsync(&h, nrm.get(), sizeof(double), cudaMemcpyDeviceToHost, s_));
-                VK_CUDA(cudaStreamSynchronize(s_));
-                const double est = std::sqrt(h); // |Q^ v| with |v| = 1
-                scal_kernel<double><<<grid1d(n), 256, 0, s_>>>(z.get(), n, nrm.get());
+            seed();
+            power_run(power, [&] {
+                const int grid = pass(dm_.q, s64_.q.get(), v.get(), z.get(), true, true);
+                power_control(power, sums.get(), nullptr, grid, false, s_);
                 std::swap(v, z);
-                if (it > 10 && std::abs(est - prev) <= 1e-6 * est) {
-                    prev = est;
-                    break;
-                }
-                prev = est;
-            }
-            lq_ = prev;
+            }, s_);
+            lq_ = estimate();
         }
         // |c^| and |b^| (scaled) for omega_0; |c| and |b| original for the KKT scales
         std::vector<double> hc(n), hrl(m), hru(m), hcs(n), hrs(m);
