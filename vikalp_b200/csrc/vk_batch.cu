@@ -56,20 +56,24 @@ struct BColEpi : EpiBase<T> {
     static constexpr bool kPerTile = CHECK;
     BCtl ctl;
     int it;
-    const int *inst, *tile_inst;
+    const int *tile_inst;
     T *x, *xbar, *xhat;
     const T *x0, *c, *l, *u;
     double *partials;
+    T tau, lam; // the tile's instance's (enter)
     struct Pre {
         T x, x0, c, l, u;
-        int b;
     };
     static constexpr bool kSkipTiles = true;
-    __device__ bool skip_tile(int t) const { return ctl.done[tile_inst[t]] != 0; }
-    __device__ Pre load(int j) const { return Pre{x[j], x0[j], c[j], l[j], u[j], inst[j]}; }
+    __device__ bool enter(int t) {
+        const int b = __ldg(tile_inst + t);
+        if (ctl.done[b] != 0) return false;
+        tau = static_cast<T>(ctl.tau[b]);
+        lam = static_cast<T>(lam_of(ctl, b, it));
+        return true;
+    }
+    __device__ Pre load(int j) const { return Pre{x[j], x0[j], c[j], l[j], u[j]}; }
     __device__ void row_pre(int j, const T (&s)[1], const Pre &p, double (&red)[NR]) const {
-        const T tau = static_cast<T>(ctl.tau[p.b]);
-        const T lam = static_cast<T>(lam_of(ctl, p.b, it));
         const T xh = clampbox(p.x - tau * (p.c + s[0]), p.l, p.u);
         xbar[j] = T(2) * xh - p.x;
         x[j] = lam * ((T(1) + T(kRhoB)) * xh - T(kRhoB) * p.x) + (T(1) - lam) * p.x0;
@@ -93,20 +97,24 @@ struct BRowEpi : EpiBase<T> {
     static constexpr bool kPerTile = CHECK;
     BCtl ctl;
     int it;
-    const int *inst, *tile_inst;
+    const int *tile_inst;
     T *y, *yhat;
     const T *y0, *rl, *ru;
     double *partials;
+    T sigma, lam; // the tile's instance's (enter)
     struct Pre {
         T y, y0, rl, ru;
-        int b;
     };
     static constexpr bool kSkipTiles = true;
-    __device__ bool skip_tile(int t) const { return ctl.done[tile_inst[t]] != 0; }
-    __device__ Pre load(int i) const { return Pre{y[i], y0[i], rl[i], ru[i], inst[i]}; }
+    __device__ bool enter(int t) {
+        const int b = __ldg(tile_inst + t);
+        if (ctl.done[b] != 0) return false;
+        sigma = static_cast<T>(ctl.sigma[b]);
+        lam = static_cast<T>(lam_of(ctl, b, it));
+        return true;
+    }
+    __device__ Pre load(int i) const { return Pre{y[i], y0[i], rl[i], ru[i]}; }
     __device__ void row_pre(int i, const T (&s)[1], const Pre &p, double (&red)[NR]) const {
-        const T sigma = static_cast<T>(ctl.sigma[p.b]);
-        const T lam = static_cast<T>(lam_of(ctl, p.b, it));
         const T v = p.y + sigma * s[0];
         const T yh = v - clampbox(v, sigma * p.rl, sigma * p.ru);
         y[i] = lam * ((T(1) + T(kRhoB)) * yh - T(kRhoB) * p.y) + (T(1) - lam) * p.y0;
@@ -136,7 +144,7 @@ struct BKktRowEpi : EpiBase<T> {
         T y, rl, ru, r;
     };
     static constexpr bool kSkipTiles = true;
-    __device__ bool skip_tile(int t) const { return ctl.done[tile_inst[t]] != 0; }
+    __device__ bool enter(int t) const { return ctl.done[tile_inst[t]] == 0; }
     __device__ Pre load(int i) const { return Pre{yhat[i], rl[i], ru[i], rs[i]}; }
     __device__ void row_pre(int, const T (&s)[1], const Pre &p, double (&red)[NR]) const {
         const double a = static_cast<double>(s[0]);
@@ -170,7 +178,7 @@ struct BKktColEpi : EpiBase<T> {
         T x, c, l, u, d;
     };
     static constexpr bool kSkipTiles = true;
-    __device__ bool skip_tile(int t) const { return ctl.done[tile_inst[t]] != 0; }
+    __device__ bool enter(int t) const { return ctl.done[tile_inst[t]] == 0; }
     __device__ Pre load(int j) const { return Pre{xhat[j], c[j], l[j], u[j], cs[j]}; }
     __device__ void row_pre(int, const T (&s)[1], const Pre &p, double (&red)[NR]) const {
         const double lam = static_cast<double>(p.c) + static_cast<double>(s[0]);
@@ -880,7 +888,6 @@ private:
         BColEpi<T, CHECK> e;
         e.ctl = c;
         e.it = it;
-        e.inst = cinst_.get();
         e.tile_inst = tinst_at_.get();
         e.x = st.x.get();
         e.xbar = st.xbar.get();
@@ -900,7 +907,6 @@ private:
         BRowEpi<T, CHECK> e;
         e.ctl = c;
         e.it = it;
-        e.inst = rinst_.get();
         e.tile_inst = tinst_a_.get();
         e.y = st.y.get();
         e.yhat = st.yhat.get();

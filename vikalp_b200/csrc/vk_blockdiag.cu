@@ -124,8 +124,8 @@ void upload_block_diag(const BlockDiag &h, DeviceBlockDiag &d, cudaStream_t s, b
     VK_CUDA(cudaMemsetAsync(d.at_val.get(), 0, padded(h.nnz) * sizeof(double), s));
     gather_values<double, double>(d.perm.get(), d.a_val.get(), d.at_val.get(), h.nnz, s);
     if (autotune) {
-        autotune_pattern<double>(d.a, d.a_val.get(), s);
-        autotune_pattern<double>(d.at, d.at_val.get(), s);
+        autotune_pattern<double>(d.a, d.a_val.get(), s, true);
+        autotune_pattern<double>(d.at, d.at_val.get(), s, true);
     }
     upload(d.rinst, h.rinst, s);
     upload(d.cinst, h.cinst, s);

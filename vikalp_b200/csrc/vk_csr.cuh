@@ -191,7 +191,7 @@ __host__ __device__ constexpr FastVariant fast_variant(int v) {
 
 template <class T, class A, int NV, class Epi, int U, bool PIPE, int MINB>
 __global__ void __launch_bounds__(kTileThreads, MINB)
-    tile_kernel_fast(CsrView<T> M, Gathers<T, NV> g, Epi epi) {
+    tile_kernel_fast(CsrView<T> M, Gathers<T, NV> g, Epi epi) { // epi: the warp's own copy (enter)
     if (epi.skip()) return;
     constexpr int NR = Epi::NR;
     static_assert(NR >= 1, "epilogues declare at least one reduction slot");
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(kTileThreads, MINB)
     };
 
     for (int tile = blockIdx.x * kWarps + warp; tile < M.ntiles; tile += gridDim.x * kWarps) {
-        if (epi.skip_tile(tile)) continue;
+        if (!epi.enter(tile)) continue;
         const int r0 = __ldg(M.tiles + tile), r1 = __ldg(M.tiles + tile + 1);
         const int k0 = __ldg(M.tile_k + tile), k1 = __ldg(M.tile_k + tile + 1);
         const int nz = k1 - k0, nrows = r1 - r0;
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(kTileThreads, MINB)
 // tile schedule, grid and epilogue interface as tile_kernel_fast.
 template <class T, class A, int NV, class Epi, int L, int U, int MINB>
 __global__ void __launch_bounds__(kTileThreads, MINB)
-    tile_kernel_sub(CsrView<T> M, Gathers<T, NV> g, Epi epi) {
+    tile_kernel_sub(CsrView<T> M, Gathers<T, NV> g, Epi epi) { // epi: the warp's own copy (enter)
     static_assert(L == 2 || L == 4 || L == 8 || L == 16 || L == 32, "sub-warp width");
     if (epi.skip()) return;
     constexpr int NR = Epi::NR;
@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(kTileThreads, MINB)
     if constexpr (Epi::kPerTile || Epi::kSkipTiles) {
         // Tile by tile (round robin): per-tile sums and skipped tiles.
         for (int tile = blockIdx.x * kWarps + warp; tile < M.ntiles; tile += gridDim.x * kWarps) {
-            if (epi.skip_tile(tile)) continue;
+            if (!epi.enter(tile)) continue;
             const int r0 = __ldg(M.tiles + tile), r1 = __ldg(M.tiles + tile + 1);
             const int k0 = __ldg(M.tile_k + tile), k1 = __ldg(M.tile_k + tile + 1);
             if (k1 - k0 > kCap)
@@ -545,7 +545,7 @@ constexpr int kRowCost = 4;
 
 template <class T, class A, int NV, class Epi, int S, int L, int U, int MINB, bool LATE>
 __global__ void __launch_bounds__(kTileThreads, MINB)
-    tile_kernel_hyb(CsrView<T> M, Gathers<T, NV> g, Epi epi) {
+    tile_kernel_hyb(CsrView<T> M, Gathers<T, NV> g, Epi epi) { // epi: the warp's own copy (enter)
     static_assert(L == 2 || L == 4 || L == 8 || L == 16, "sub-warp width");
     if (epi.skip()) return;
     constexpr int NR = Epi::NR;
@@ -679,7 +679,7 @@ __global__ void __launch_bounds__(kTileThreads, MINB)
     const int wid = blockIdx.x * kWarps + warp;
     if constexpr (Epi::kPerTile || Epi::kSkipTiles) {
         for (int tile = wid; tile < M.ntiles; tile += W) {
-            if (epi.skip_tile(tile)) continue;
+            if (!epi.enter(tile)) continue;
             const int r0 = __ldg(M.tiles + tile), r1 = __ldg(M.tiles + tile + 1);
             for (int rb = r0; rb < r1; rb += 32) {
                 const int re = rb + 32 < r1 ? rb + 32 : r1;
@@ -1072,16 +1072,18 @@ template <class A>
 struct EpiBase {
     static constexpr int NR = 1;
     // kPerTile: after each warp-tile the warp's reductions are summed and
-    // passed to tile_done(tile, red) (FAST order only); skip_tile(tile) lets
-    // a pass leave whole tiles untouched.
+    // passed to tile_done(tile, red) (FAST order only). enter(tile), called by
+    // a warp before each of its tiles, lets a pass leave the tile untouched
+    // (false) and fetch what all of its rows share (into the epilogue's own
+    // members: every thread has its copy).
     static constexpr bool kPerTile = false;
-    static constexpr bool kSkipTiles = false; // true when skip_tile is overridden
+    static constexpr bool kSkipTiles = false; // true when enter is overridden
     struct Pre {};
     __device__ Pre load(int) const { return Pre{}; }
     __device__ A init(int, int) const { return A(0); }
     __device__ A gscale(int) const { return A(1); }
     __device__ bool skip() const { return false; }
-    __device__ bool skip_tile(int) const { return false; }
+    __device__ bool enter(int) { return true; }
     template <int NR>
     __device__ void tile_done(int, double (&)[NR]) const {}
     template <int NR>
@@ -1139,12 +1141,13 @@ void convert_values(const TS *src, TD *dst, int64_t n, cudaStream_t s);
 void expand_rows(const CsrPattern32 &p, int *rowidx, cudaStream_t s);
 // Autotuner: times every FAST kernel variant on this matrix (a plain product
 // into scratch vectors, a few launches each) and stores the fastest in
-// p.variant. Matrices below `min_nnz` keep variant 0.
+// p.variant. Matrices below `min_nnz` keep variant 0. tiles: the pattern's
+// passes go tile by tile (batches).
 // The environment variable VIKALP_B200_VARIANT=<v> (0 <= v < kFastVariants)
 // pins every pattern (and every tuned pass) to variant v instead, at any size:
 // a knob for tests that run whole solves on each kernel variant.
 template <class T>
-void autotune_pattern(CsrPattern32 &p, const T *val, cudaStream_t s, int64_t min_nnz = 200000);
+void autotune_pattern(CsrPattern32 &p, const T *val, cudaStream_t s, bool tiles = false, int64_t min_nnz = 200000);
 // The pinned variant, or -1.
 int forced_variant();
 
