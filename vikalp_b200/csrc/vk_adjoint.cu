@@ -532,17 +532,18 @@ public:
     AdjointEngine(const vk_problem *probs, int count, const vk_adjoint_options &o) : o_(o), B_(count) {
         VK_CUDA(cudaSetDevice(o.device));
         device_error_flag();
-        VK_CUDA(cudaStreamCreateWithFlags(&s_, cudaStreamNonBlocking));
+        s_.create();
+        PoolScope pool(s_);
         concat_instances(probs, count, h_);
         upload_block_diag(h_, d_, s_, false);
     }
     ~AdjointEngine() {
         if (g_) cudaGraphExecDestroy(g_);
-        if (s_) cudaStreamDestroy(s_);
     }
 
     void run(const double *x, const double *y, const double *g, double w_obj, double *dc, double *db, double *da,
              vk_adjoint_info *info) {
+        PoolScope pool(s_);
         const int m = h_.m, n = h_.n, B = B_;
         const int mm = std::max(m, 1);
         DevBuf<double> dx(n), dy(mm), dg(n), l(n), u(n), rl(mm), ru(mm);
@@ -755,9 +756,9 @@ private:
         return ex;
     }
 
+    OwnStream s_; // first: outlives the buffers
     vk_adjoint_options o_;
     int B_;
-    cudaStream_t s_ = nullptr;
     BlockDiag h_;
     DeviceBlockDiag d_;
     DevBuf<double> rmask_, fmask_, ubar_, vbar_, w_, dir_;

@@ -399,7 +399,8 @@ public:
     BatchEngine(const vk_problem *probs, int count, const vk_options &o) : o_(o), B_(count) {
         VK_CUDA(cudaSetDevice(o.device));
         device_error_flag();
-        VK_CUDA(cudaStreamCreateWithFlags(&s_, cudaStreamNonBlocking));
+        s_.create();
+        PoolScope pool(s_);
         mixed_ = o.precision == VK_PREC_MIXED;
         chunk_ = std::max(2, o.check_every > 0 ? o.check_every : 64);
         log_.stream(s_);
@@ -412,10 +413,10 @@ public:
     ~BatchEngine() {
         if (g64_) cudaGraphExecDestroy(g64_);
         if (g32_) cudaGraphExecDestroy(g32_);
-        if (s_) cudaStreamDestroy(s_);
     }
 
     void solve(vk_result *results) {
+        PoolScope pool(s_);
         const auto started = std::chrono::steady_clock::now();
         reset_control();
         cudaEvent_t e0, e1;
@@ -943,10 +944,10 @@ private:
         launch_tiles<T, T, 1, false>(view(at_, st.kat.get()), Gathers<T, 1>{{yg}}, k, s_);
     }
 
+    OwnStream s_; // first: outlives the buffers
     vk_options o_;
     int B_;
     PhaseLog log_{o_.verbose, "batch", nullptr};
-    cudaStream_t s_ = nullptr;
     bool mixed_ = false;
     int chunk_ = 64;
     int m_ = 0, n_ = 0;
@@ -1510,6 +1511,7 @@ public:
         m_ = base_.m_;
         n_ = base_.n_;
         s_ = base_.s_;
+        PoolScope pool(s_);
         mixed_ = o.precision == VK_PREC_MIXED;
         chunk_ = base_.chunk_;
         const int width = B_ >= 128 ? 128 : 32;
@@ -1537,6 +1539,7 @@ public:
     }
 
     void solve(const double *lower, const double *upper, const double *warm, vk_result *results) {
+        PoolScope pool(s_);
         const auto started = std::chrono::steady_clock::now();
         PhaseLog lg(o_.verbose, "shared", s_);
         const int n = n_, m = m_;

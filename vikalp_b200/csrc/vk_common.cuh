@@ -38,7 +38,56 @@ struct Unsupported : std::runtime_error {
 
 #define VK_LAUNCH_CHECK() VK_CUDA(cudaGetLastError())
 
-// Owning device buffer (cudaMalloc / cudaFree). Size in elements.
+// Device memory of the library's own solves (vk_pool.cu): a memory pool per
+// device, separate from the application's, that keeps up to kPoolKeep unused
+// bytes for the next call; the driver takes them back when an allocation of
+// the process needs them. A call on a batch makes ~200 allocations; cudaMalloc
+// and cudaFree took 5-25 ms of it, and up to a second when the host was busy.
+constexpr unsigned long long kPoolKeep = 2ull << 30;
+void *pool_alloc(size_t bytes, cudaStream_t s); // ordered on s
+void pool_free(void *p, cudaStream_t s) noexcept;
+
+// While a PoolScope lives, its thread's DevBufs come from the pool, ordered on
+// the scope's stream: for code whose buffers are used on that one stream. A
+// buffer remembers its stream (which must outlive it) and returns to the pool
+// in that stream's order, from whichever thread. Elsewhere (operators and vectors
+// that callers use on streams of their own) DevBuf is cudaMalloc / cudaFree.
+struct PoolMode {
+    bool on = false;
+    cudaStream_t stream = nullptr;
+};
+inline PoolMode &pool_mode() {
+    static thread_local PoolMode mode;
+    return mode;
+}
+class PoolScope {
+public:
+    explicit PoolScope(cudaStream_t s) : before_(pool_mode()) { pool_mode() = PoolMode{true, s}; }
+    ~PoolScope() { pool_mode() = before_; }
+    PoolScope(const PoolScope &) = delete;
+    PoolScope &operator=(const PoolScope &) = delete;
+
+private:
+    PoolMode before_;
+};
+
+// A non-blocking stream that outlives the buffers declared after it.
+class OwnStream {
+public:
+    OwnStream() = default;
+    ~OwnStream() {
+        if (s_) cudaStreamDestroy(s_);
+    }
+    OwnStream(const OwnStream &) = delete;
+    OwnStream &operator=(const OwnStream &) = delete;
+    void create() { VK_CUDA(cudaStreamCreateWithFlags(&s_, cudaStreamNonBlocking)); }
+    operator cudaStream_t() const { return s_; }
+
+private:
+    cudaStream_t s_ = nullptr;
+};
+
+// Owning device buffer (PoolScope, or cudaMalloc / cudaFree). Size in elements.
 template <class T>
 class DevBuf {
 public:
@@ -47,22 +96,34 @@ public:
     ~DevBuf() { release(); }
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
-    DevBuf(DevBuf &&o) noexcept : p_(std::exchange(o.p_, nullptr)), n_(std::exchange(o.n_, 0)) {}
+    DevBuf(DevBuf &&o) noexcept : p_(std::exchange(o.p_, nullptr)), n_(std::exchange(o.n_, 0)), from_(o.from_) {}
     DevBuf &operator=(DevBuf &&o) noexcept {
         if (this != &o) {
             release();
             p_ = std::exchange(o.p_, nullptr);
             n_ = std::exchange(o.n_, 0);
+            from_ = o.from_;
         }
         return *this;
     }
     void reset(size_t n) {
         release();
-        if (n > 0) VK_CUDA(cudaMalloc(reinterpret_cast<void **>(&p_), n * sizeof(T)));
+        from_ = pool_mode();
+        if (n > 0) {
+            if (from_.on)
+                p_ = static_cast<T *>(pool_alloc(n * sizeof(T), from_.stream));
+            else
+                VK_CUDA(cudaMalloc(reinterpret_cast<void **>(&p_), n * sizeof(T)));
+        }
         n_ = n;
     }
     void release() noexcept {
-        if (p_) cudaFree(p_);
+        if (p_) {
+            if (from_.on)
+                pool_free(p_, from_.stream);
+            else
+                cudaFree(p_);
+        }
         p_ = nullptr;
         n_ = 0;
     }
@@ -73,6 +134,7 @@ public:
 private:
     T *p_ = nullptr;
     size_t n_ = 0;
+    PoolMode from_;
 };
 
 // Pinned host buffer.

@@ -460,7 +460,8 @@ struct QcEpi : EpiRow<double, QcEpi> {
 Solver::Solver(const vk_problem &p, const vk_options &o) : opts_(o) {
     VK_CUDA(cudaSetDevice(o.device));
     device_error_flag(); // allocated here, never inside a graph capture
-    VK_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
+    stream_.create();
+    PoolScope pool(stream_);
     PhaseLog log(o.verbose, "create", stream_);
     dm_ = upload_model(p, stream_, o.verbose, o.spmv_order == VK_SPMV_FAST);
     log.mark("upload + transpose");
@@ -492,6 +493,7 @@ std::string Solver::set_options(const vk_options &o) {
 
 bool Solver::profile(long long iterations, vk_pass_profile *out) {
     VK_CUDA(cudaSetDevice(opts_.device));
+    PoolScope pool(stream_);
     PassProfile pp;
     if (!engine_->profile(iterations, pp)) return false;
     *out = vk_pass_profile{};
@@ -508,7 +510,6 @@ bool Solver::profile(long long iterations, vk_pass_profile *out) {
 Solver::~Solver() {
     engine_.reset();
     dm_.reset();
-    if (stream_) cudaStreamDestroy(stream_);
 }
 
 namespace {
@@ -518,6 +519,23 @@ __global__ void fill_override_kernel(const double *__restrict__ ov, const double
                                      const int *__restrict__ perm, int n, double *__restrict__ out) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j < n) out[j] = ov ? ov[perm ? perm[j] : j] : model[j];
+}
+
+// The checks of a solve's inputs (continuous_common.hpp:80-110, pdhg.cpp:29-33)
+// on the device; bits of *found in the order the reference tests them.
+enum : int { kNanOverride = 1, kBadInterval = 2, kBadWarm = 4 };
+__global__ void check_inputs_kernel(const double *__restrict__ ov_lo, const double *__restrict__ ov_hi,
+                                    const double *__restrict__ lo, const double *__restrict__ hi,
+                                    const double *__restrict__ warm, int n, int *__restrict__ found) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    int bad = 0;
+    if (j < n) {
+        if ((ov_lo && isnan(ov_lo[j])) || (ov_hi && isnan(ov_hi[j]))) bad |= kNanOverride;
+        if (isnan(lo[j]) || isnan(hi[j]) || lo[j] > hi[j]) bad |= kBadInterval;
+        if (warm && !isfinite(warm[j])) bad |= kBadWarm;
+    }
+    for (int o = 16; o > 0; o >>= 1) bad |= __shfl_xor_sync(0xffffffffu, bad, o);
+    if (bad != 0 && (threadIdx.x & 31) == 0) atomicOr(found, bad);
 }
 } // namespace
 
@@ -536,31 +554,34 @@ void Solver::solve(const double *warm, const double *lo_ovr, const double *hi_ov
         r->status = VK_STATUS_INVALID_MODEL;
         std::snprintf(r->message, sizeof(r->message), "%s", msg);
     };
-    // copy_bounds (continuous_common.hpp:80-110)
-    for (const double *ov : {lo_ovr, hi_ovr}) {
-        if (!ov) continue;
-        for (int j = 0; j < n; ++j)
-            if (std::isnan(ov[j])) return fail("variable bound overrides must be empty or sized and non-NaN");
-    }
-    for (int j = 0; j < n; ++j) {
-        const double l = lo_ovr ? lo_ovr[j] : dm.h_vl[j];
-        const double u = hi_ovr ? hi_ovr[j] : dm.h_vu[j];
-        if (std::isnan(l) || std::isnan(u) || l > u) return fail("variable bound overrides contain an invalid interval");
-    }
-    // warm start (pdhg.cpp:29-33)
-    if (warm)
-        for (int j = 0; j < n; ++j)
-            if (!std::isfinite(warm[j])) return fail("warm start must be empty or finite and sized to the model");
-
     cudaStream_t s = stream_;
+    PoolScope pool(s);
     DevBuf<double> lo(n), hi(n), dwarm(warm ? n : 0), ov_lo(lo_ovr ? n : 0), ov_hi(hi_ovr ? n : 0);
-    if (lo_ovr) VK_CUDA(cudaMemcpyAsync(ov_lo.get(), lo_ovr, n * sizeof(double), cudaMemcpyHostToDevice, s));
-    if (hi_ovr) VK_CUDA(cudaMemcpyAsync(ov_hi.get(), hi_ovr, n * sizeof(double), cudaMemcpyHostToDevice, s));
-    if (warm) VK_CUDA(cudaMemcpyAsync(dwarm.get(), warm, n * sizeof(double), cudaMemcpyHostToDevice, s));
+    const auto up = [&](DevBuf<double> &d, const double *h) {
+        if (!h) return;
+        if (n * sizeof(double) >= kStageMin)
+            stage_h2d(d.get(), h, n * sizeof(double), s);
+        else
+            VK_CUDA(cudaMemcpyAsync(d.get(), h, n * sizeof(double), cudaMemcpyHostToDevice, s));
+    };
+    up(ov_lo, lo_ovr);
+    up(ov_hi, hi_ovr);
+    up(dwarm, warm);
     const int *cperm = dm.reordered() ? dm.cperm.get() : nullptr;
     fill_override_kernel<<<grid1d(n), 256, 0, s>>>(lo_ovr ? ov_lo.get() : nullptr, dm.vl.get(), cperm, n, lo.get());
     fill_override_kernel<<<grid1d(n), 256, 0, s>>>(hi_ovr ? ov_hi.get() : nullptr, dm.vu.get(), cperm, n, hi.get());
     VK_LAUNCH_CHECK();
+    DevBuf<int> found(1);
+    VK_CUDA(cudaMemsetAsync(found.get(), 0, sizeof(int), s));
+    check_inputs_kernel<<<grid1d(n), 256, 0, s>>>(ov_lo.get(), ov_hi.get(), lo.get(), hi.get(), dwarm.get(), n,
+                                                  found.get());
+    VK_LAUNCH_CHECK();
+    int bad = 0;
+    VK_CUDA(cudaMemcpyAsync(&bad, found.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
+    VK_CUDA(cudaStreamSynchronize(s));
+    if (bad & kNanOverride) return fail("variable bound overrides must be empty or sized and non-NaN");
+    if (bad & kBadInterval) return fail("variable bound overrides contain an invalid interval");
+    if (bad & kBadWarm) return fail("warm start must be empty or finite and sized to the model");
     DevBuf<double> dwarm_dev(warm && cperm ? n : 0); // the warm start in the device's column order
     if (warm && cperm) gather_values<double, double>(cperm, dwarm.get(), dwarm_dev.get(), n, s);
     const double *warm_dev = !warm ? nullptr : cperm ? dwarm_dev.get() : dwarm.get();
@@ -643,15 +664,15 @@ void Solver::solve(const double *warm, const double *lo_ovr, const double *hi_ov
             vud_out = back.get() + 2 * static_cast<size_t>(n);
         }
     }
-    std::vector<double> hx(n);
-    stage_d2h(hx.data(), x_out, n * sizeof(double), s);
+    std::vector<double> own(r->x ? 0 : n); // x, where the caller has no room for it (the objective needs it)
+    double *hx = r->x ? r->x : own.data();
+    stage_d2h(hx, x_out, n * sizeof(double), s);
     if (r->y && m > 0) stage_d2h(r->y, yo.get(), m * sizeof(double), s);
     if (r->row_lower_dual && m > 0) stage_d2h(r->row_lower_dual, ld.get(), m * sizeof(double), s);
     if (r->row_upper_dual && m > 0) stage_d2h(r->row_upper_dual, ud.get(), m * sizeof(double), s);
     if (r->var_lower_dual) stage_d2h(r->var_lower_dual, vld_out, n * sizeof(double), s);
     if (r->var_upper_dual) stage_d2h(r->var_upper_dual, vud_out, n * sizeof(double), s);
     VK_CUDA(cudaStreamSynchronize(s));
-    if (r->x) std::memcpy(r->x, hx.data(), n * sizeof(double));
 
     // objective: offset + c'x (+ 0.5 x'Qx), the reference's order (continuous_common.hpp:284-300)
     double dot = 0.0;

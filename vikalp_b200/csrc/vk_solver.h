@@ -64,8 +64,8 @@ public:
     cudaStream_t stream() const { return stream_; }
 
 private:
+    OwnStream stream_; // first: outlives the buffers
     vk_options opts_;
-    cudaStream_t stream_ = nullptr;
     std::unique_ptr<DeviceModel> dm_;
     std::unique_ptr<Engine> engine_;
 };

@@ -20,7 +20,7 @@
 namespace vk {
 
 constexpr size_t kStageChunk = size_t(4) << 20; // bytes per staged chunk (and per pinned buffer)
-constexpr size_t kStageMin = size_t(16) << 20;  // smaller transfers are not staged
+constexpr size_t kStageMin = size_t(8) << 20;   // smaller transfers are not staged
 constexpr int kStageThreads = 4;
 // Device -> host copies write into the caller's memory, which is often fresh
 // (a first touch faults each page in); the kernel serves page faults on
