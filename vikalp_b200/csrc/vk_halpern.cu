@@ -700,7 +700,7 @@ private:
     }
 
     // A model whose matrices fit the GPU's shared memory iterates there
-    // (vk_resident.cuh): 11.0 us an iteration against 23.7 for the passes at
+    // (vk_resident.cuh): 10.3 us an iteration against 23.7 for the passes at
     // 600,000 nonzeros, 16.1 against 37.5 at 720,000 (float64; past about
     // 800,000 they no longer fit), 17.5 against 26.4 at 940,000 (float32).
     void plan_resident() {

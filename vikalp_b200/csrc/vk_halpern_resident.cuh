@@ -95,7 +95,6 @@ __global__ void __launch_bounds__(kRsThreads, 1) rs_halpern_kernel(RsHalArgs<T> 
     // qx = Q^ x over the own columns (QP)
     const auto q_pass = [&] {
         rs_products(sq, A.x, prod);
-        __syncthreads();
         rs_rows(sq, prod, [&](int j, T sum) { qx[j] = sum; });
         __syncthreads();
     };
@@ -104,6 +103,12 @@ __global__ void __launch_bounds__(kRsThreads, 1) rs_halpern_kernel(RsHalArgs<T> 
         if (!bar.sync()) return; // x is read everywhere before anyone writes it
     }
 
+    struct ColIn {
+        T x, x0, c, l, u;
+    };
+    struct RowIn {
+        T y, y0, lo, hi;
+    };
     for (int ch = 0; ch < A.chunks; ++ch) {
         const T tau = static_cast<T>(c.tau), sigma = static_cast<T>(c.sigma), rho = static_cast<T>(c.rho);
         const double kb = static_cast<double>(c.k_base);
@@ -117,13 +122,12 @@ __global__ void __launch_bounds__(kRsThreads, 1) rs_halpern_kernel(RsHalArgs<T> 
             const T lam = lams[it % kTab];
             const bool check = it == A.chunk - 1;
             rs_products(st, A.y, prod);
-            __syncthreads();
-            rs_rows(st, prod, [&](int j, T sum) {
-                const T xv = x[j], xz = x0[j];
-                const T g = QP ? cc[j] + qx[j] + sum : cc[j] + sum;
-                const T xh = clampbox(xv - tau * g, l[j], u[j]);
-                const T xn = lam * ((T(1) + rho) * xh - rho * xv) + (T(1) - lam) * xz;
+            const auto column = [&](int j) { return ColIn{x[j], x0[j], QP ? cc[j] + qx[j] : cc[j], l[j], u[j]}; };
+            rs_rows(st, prod, column, [&](int j, T sum, const ColIn &p) {
+                const T xv = p.x, xz = p.x0;
+                const T xh = clampbox(xv - tau * (p.c + sum), p.l, p.u);
                 A.xbar[c0 + j] = T(2) * xh - xv;
+                const T xn = lam * ((T(1) + rho) * xh - rho * xv) + (T(1) - lam) * xz;
                 x[j] = xn;
                 if (QP) A.x[c0 + j] = xn;
                 if (check) {
@@ -136,11 +140,11 @@ __global__ void __launch_bounds__(kRsThreads, 1) rs_halpern_kernel(RsHalArgs<T> 
             });
             if (!bar.sync()) return;
             rs_products(sa, A.xbar, prod);
-            __syncthreads();
-            rs_rows(sa, prod, [&](int i, T sum) {
-                const T yv = y[i], yz = y0[i];
+            const auto dual = [&](int i) { return RowIn{y[i], y0[i], sigma * rl[i], sigma * ru[i]}; };
+            rs_rows(sa, prod, dual, [&](int i, T sum, const RowIn &p) {
+                const T yv = p.y, yz = p.y0;
                 const T v = yv + sigma * sum;
-                const T yh = v - clampbox(v, sigma * rl[i], sigma * ru[i]);
+                const T yh = v - clampbox(v, p.lo, p.hi);
                 const T yn = lam * ((T(1) + rho) * yh - rho * yv) + (T(1) - lam) * yz;
                 A.y[r0 + i] = yn;
                 y[i] = yn;
@@ -161,19 +165,16 @@ __global__ void __launch_bounds__(kRsThreads, 1) rs_halpern_kernel(RsHalArgs<T> 
         // the check: K x^, (Q^ x^,) K'y^
         double s[kCheckSums] = {dx2, dx0, dy2, dy0};
         rs_products(sa, A.xhat, prod64);
-        __syncthreads();
         rs_rows(sa, prod64, [&](int i, double sum) {
             kkt_row_terms(sum, rl[i], ru[i], A.rs[r0 + i], A.yhat[r0 + i], s + kColCheckSums + kRowCheckSums);
         });
         __syncthreads();
         if (QP) {
             rs_products(sq, A.xhat, prod64);
-            __syncthreads();
             rs_rows(sq, prod64, [&](int j, double sum) { qh[j] = static_cast<T>(sum); });
             __syncthreads();
         }
         rs_products(st, A.yhat, prod64);
-        __syncthreads();
         rs_rows(st, prod64, [&](int j, double sum) {
             kkt_col_terms(sum, cc[j], QP ? static_cast<double>(qh[j]) : 0.0, A.cs[c0 + j], l[j], u[j], A.xhat[c0 + j],
                           s + kCheckSums - kKktColSums);

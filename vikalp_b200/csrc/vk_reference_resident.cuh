@@ -138,22 +138,29 @@ __global__ void __launch_bounds__(kRsThreads, 1) rs_reference_kernel(RsRefArgs A
         cycles[q] += now - mark;
         mark = now;
     };
+    struct ColIn {
+        double x, c, l, u;
+    };
+    struct RowIn {
+        double y, kx, lo, hi;
+    };
     for (;; ++k) {
         // K'y_k, the stationarity of iteration k-1, and the primal step of
         // iteration k unless the control step may still change tau
         const bool policy = ref_policy_iter(k);
         const double tau = c.tau;
         rs_products(st, A.y, prod);
-        __syncthreads();
         double top = 0.0;
-        rs_rows(st, prod, [&](int j, double sum) {
-            const double xv = x[j], lo = l[j], hi = u[j];
+        const auto column = [&](int j) { return ColIn{x[j], cc[j], l[j], u[j]}; };
+        rs_rows(st, prod, column, [&](int j, double sum, const ColIn &p) {
+            if (policy)
+                aty[j] = sum;
+            else
+                A.xn[c0 + j] = xn[j] = ref_primal(tau, sum, p.x, p.c, p.l, p.u);
             if (k >= 1) {
-                const double px = clampbox(__dadd_rn(-__dadd_rn(sum, cc[j]), xv), lo, hi);
-                top = smax(top, fabs(__dadd_rn(-px, xv)));
+                const double px = clampbox(__dadd_rn(-__dadd_rn(sum, p.c), p.x), p.l, p.u);
+                top = smax(top, fabs(__dadd_rn(-px, p.x)));
             }
-            aty[j] = sum;
-            if (!policy) A.xn[c0 + j] = xn[j] = ref_primal(tau, sum, xv, cc[j], lo, hi);
         });
         if (!bar.sync_max(top, warps, rd + (k & 3))) return;
         lap(0);
@@ -182,7 +189,7 @@ __global__ void __launch_bounds__(kRsThreads, 1) rs_reference_kernel(RsRefArgs A
             c.rd = __ldcg(rd + (k & 3));
             ref_decide(c);
         }
-        __syncthreads();
+        __syncthreads(); // c
         if (c.done) { // x_k, y_k are the answer
             if (blockIdx.x == 0 && tid == 0) *A.ctl = c;
             break;
@@ -192,14 +199,14 @@ __global__ void __launch_bounds__(kRsThreads, 1) rs_reference_kernel(RsRefArgs A
         const double sigma = c.sigma, inv = c.inv_sigma;
         const bool restart = c.restart != 0;
         top = 0.0;
-        rs_rows(sa, prod, [&](int i, double kxn) {
-            const double lo = rl[i], hi = ru[i];
-            const double kxbar = restart ? kxn : __dadd_rn(__dmul_rn(2.0, kxn), -kx[i]);
-            kx[i] = kxn;
-            const double yarg = __dadd_rn(__dmul_rn(sigma, kxbar), y[i]);
-            const double yp = clampbox(__dmul_rn(inv, yarg), lo, hi);
+        const auto dual = [&](int i) { return RowIn{y[i], kx[i], rl[i], ru[i]}; };
+        rs_rows(sa, prod, dual, [&](int i, double kxn, const RowIn &p) {
+            const double kxbar = restart ? kxn : __dadd_rn(__dmul_rn(2.0, kxn), -p.kx);
+            const double yarg = __dadd_rn(__dmul_rn(sigma, kxbar), p.y);
+            const double yp = clampbox(__dmul_rn(inv, yarg), p.lo, p.hi);
             A.y[r0 + i] = y[i] = __dadd_rn(__dmul_rn(-sigma, yp), yarg);
-            top = smax(top, fabs(__dadd_rn(clampbox(kxn, lo, hi), -kxn)));
+            kx[i] = kxn;
+            top = smax(top, fabs(__dadd_rn(clampbox(kxn, p.lo, p.hi), -kxn)));
         });
         if (!bar.sync_max(top, warps, rp + (k & 3))) return;
         lap(2);

@@ -42,6 +42,7 @@ struct RsSide {
     const I *idx;
     const int *ro;
     int rows, nnz, L;
+    bool longs; // some row goes to a whole warp
 };
 
 template <class T, class I>
@@ -52,11 +53,15 @@ __device__ RsSide<T, I> rs_load(const int *__restrict__ ro, const int *__restric
         v[k] = __ldg(val + k0 + k);
         idx[k] = static_cast<I>(__ldg(ci + k0 + k));
     }
-    for (int r = threadIdx.x; r <= rows; r += blockDim.x) sro[r] = ro[r0 + r] - k0;
     // lanes per row: every thread busy in one round, at most about one per nonzero
     int L = 1;
     while (L < 32 && rows * L * 2 <= static_cast<int>(blockDim.x) && rows * L < nnz) L *= 2;
-    return RsSide<T, I>{v, idx, sro, rows, nnz, L};
+    bool lone = false;
+    for (int r = threadIdx.x; r <= rows; r += blockDim.x) {
+        sro[r] = ro[r0 + r] - k0;
+        lone = lone || (r < rows && ro[r0 + r + 1] - ro[r0 + r] > kRsWarpRow * L);
+    }
+    return RsSide<T, I>{v, idx, sro, rows, nnz, L, __syncthreads_or(lone) != 0};
 }
 
 // prod[k] = v_k x[idx_k]; x is written by other CTAs during the launch. A:
@@ -84,33 +89,66 @@ __device__ __forceinline__ void rs_products(const RsSide<T, I> &s, const T *x, A
     }
 }
 
-// row(r, sum) for every row, in one lane of the row's group.
-template <class A, class T, class I, class F>
-__device__ __forceinline__ void rs_rows(const RsSide<T, I> &s, const A *prod, F &&row) {
+// The sum over a group of L lanes, in every one of them.
+template <class A>
+__device__ __forceinline__ A rs_group_sum(A v, int L) {
+    const unsigned FULL = 0xffffffffu;
+    if (L > 16) v += __shfl_xor_sync(FULL, v, 16);
+    if (L > 8) v += __shfl_xor_sync(FULL, v, 8);
+    if (L > 4) v += __shfl_xor_sync(FULL, v, 4);
+    if (L > 2) v += __shfl_xor_sync(FULL, v, 2);
+    if (L > 1) v += __shfl_xor_sync(FULL, v, 1);
+    return v;
+}
+
+// Waits for the block's products, then row(r, sum, pre(r)) for every row, in
+// one lane of the row's group; the first rows' bounds and pre(r) are fetched
+// before the wait (2,000 x 5,000 LP 5.36 -> 5.17 us an iteration, 50,000 x
+// 100,000 10.63 -> 10.31).
+template <class A, class T, class I, class P, class F>
+__device__ __forceinline__ void rs_rows(const RsSide<T, I> &s, const A *prod, P &&pre, F &&row) {
     const unsigned FULL = 0xffffffffu;
     const int L = s.L, lane = threadIdx.x & 31, sl = lane & (L - 1);
-    const int first = (static_cast<int>(threadIdx.x) & ~31) / L; // the warp's first row: uniform trip count
-    for (int rb = first; rb < s.rows; rb += static_cast<int>(blockDim.x) / L) {
-        const int r = rb + lane / L;
-        const bool valid = r < s.rows;
-        const int a = valid ? s.ro[r] : 0, b = valid ? s.ro[r + 1] : 0;
-        const bool lone = b - a > kRsWarpRow * L; // summed by the whole warp below
+    const int step = static_cast<int>(blockDim.x) / L;
+    int r = static_cast<int>(threadIdx.x) / L;
+    int rb = (static_cast<int>(threadIdx.x) & ~31) / L; // the warp's first row: uniform trip count
+    bool valid = r < s.rows;
+    int a = valid ? s.ro[r] : 0, b = valid ? s.ro[r + 1] : 0;
+    decltype(pre(0)) in{};
+    if (valid) in = pre(r);
+    __syncthreads();
+    while (rb < s.rows) {
         A acc = A(0);
+        const bool lone = s.longs && b - a > kRsWarpRow * L; // summed by the whole warp below
         if (!lone)
             for (int k = a + sl; k < b; k += L) acc += prod[k];
-        for (int o = L >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(FULL, acc, o);
-        unsigned lm = __ballot_sync(FULL, lone && sl == 0);
-        while (lm) {
-            const int src = __ffs(lm) - 1;
-            const int fa = __shfl_sync(FULL, a, src), fb = __shfl_sync(FULL, b, src);
-            A part = A(0);
-            for (int k = fa + lane; k < fb; k += 32) part += prod[k];
-            part = warp_sum(part);
-            if (lane == src) acc = part;
-            lm &= lm - 1u;
+        acc = rs_group_sum(acc, L);
+        if (s.longs) {
+            unsigned lm = __ballot_sync(FULL, lone && sl == 0);
+            while (lm) {
+                const int src = __ffs(lm) - 1;
+                const int fa = __shfl_sync(FULL, a, src), fb = __shfl_sync(FULL, b, src);
+                A part = A(0);
+                for (int k = fa + lane; k < fb; k += 32) part += prod[k];
+                part = warp_sum(part);
+                if (lane == src) acc = part;
+                lm &= lm - 1u;
+            }
         }
-        if (valid && sl == 0) row(r, acc);
+        if (valid && sl == 0) row(r, acc, in);
+        rb += step;
+        r += step;
+        if (rb >= s.rows) break;
+        valid = r < s.rows;
+        a = valid ? s.ro[r] : 0;
+        b = valid ? s.ro[r + 1] : 0;
+        if (valid) in = pre(r);
     }
+}
+// The same for rows without inputs.
+template <class A, class T, class I, class F>
+__device__ __forceinline__ void rs_rows(const RsSide<T, I> &s, const A *prod, F &&row) {
+    rs_rows(s, prod, [](int) { return 0; }, [&](int r, A sum, int) { row(r, sum); });
 }
 
 // A CTA's block barrier at the end of a gather: false when any of its threads
@@ -197,10 +235,10 @@ bool rs_plan(const CsrPattern32 &a, const CsrPattern32 &at, const CsrPattern32 *
 
 // CTAs (at most one per SM) and threads for `nnz` nonzeros. Timed per
 // iteration (float64 Halpern, 37 / 74 / 148 CTAs x 256 / 512 / 768 / 1024
-// threads): 4,000 nonzeros 4.8 us with 37 x 256 (148 x 1024: 5.3), 40,000
-// nonzeros 5.4 us with 148 x 256 (37 x 256: 6.5, 148 x 1024: 5.8), 120,000
-// nonzeros 6.4 us with 148 x 512 (256: 7.3, 1024: 6.8), 600,000 nonzeros 11.0
-// us with 148 x 768 (256: 13.5, 1024: 11.5).
+// threads): 4,000 nonzeros 4.6 us with 31 x 256 (148 x 1024: 5.3), 40,000
+// nonzeros 5.2 us with 148 x 256 (37 x 256: 6.5, 148 x 1024: 5.5), 120,000
+// nonzeros 6.0 us with 148 x 512 (256: 6.4, 1024: 6.5), 600,000 nonzeros 10.3
+// us with 148 x 768 (256: 12.2, 1024: 10.9).
 int rs_grid(int64_t nnz);
 int rs_threads(int64_t nnz, int grid);
 
