@@ -241,6 +241,33 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
                  : "memory");
 }
 
+// ---------------------------------------------------------------------------
+// Programmatic dependent launch. A kernel launched by launch_after starts while
+// the kernel before it on the stream drains (its CTAs take slots as they come
+// free) and calls pdl_wait before it touches anything; that returns once the
+// kernel before it has completed, so nothing else changes for either. Saves the
+// launch gap between the passes of an iteration.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void pdl_wait() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <class K, class... A>
+inline void launch_after(K kernel, int grid, int threads, size_t smem, cudaStream_t s, const A &...args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(grid));
+    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    VK_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+}
+
 // Codes a kernel writes to the device error flag (first one wins).
 enum DeviceError : int { kDevErrNone = 0, kDevErrBarrierTimeout = 1 };
 

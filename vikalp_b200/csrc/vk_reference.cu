@@ -247,6 +247,7 @@ struct StoreEpi : EpiRow<double, StoreEpi> {
 
 // The control step (ref_decide). One thread.
 __global__ void ref_control_kernel(RefCtl *ctl) {
+    pdl_wait();
     RefCtl c = *ctl;
     if (c.done) return;
     ref_decide(c);
@@ -608,7 +609,7 @@ private:
             tiles(view(dm_.at, kat_.get()), Gathers<double, 1>{{y_.get()}}, e);
         }
         mark(1);
-        ref_control_kernel<<<1, 1, 0, s_>>>(ctl_.get());
+        launch_after(ref_control_kernel, 1, 1, 0, s_, ctl_.get());
         VK_LAUNCH_CHECK();
         if (dm_.qp)
             ref_primal_kernel<true><<<grid1d(n), 256, 0, s_>>>(ctl_.get(), cur, aty_.get(), sc_.get(), qx_.get(),
@@ -651,7 +652,7 @@ private:
             tiles(col_view(), Gathers<double, 1>{{y_.get()}}, e);
         }
         mark(1);
-        ref_control_kernel<<<1, 1, 0, s_>>>(ctl_.get());
+        launch_after(ref_control_kernel, 1, 1, 0, s_, ctl_.get());
         VK_LAUNCH_CHECK();
         if (k % 50 == 1) {
             if (dm_.qp)
