@@ -1,6 +1,7 @@
-"""Solves whose model iterates in the GPU's shared memory (vk_resident.cuh)
-against the NumPy restatement, at the shapes where its partition, its lanes
-per row and its launches have edges: one row and column, empty rows and
+"""Solves whose model iterates in the shared memory of one cluster or of the GPU
+(vk_halpern_cluster.cuh, vk_resident.cuh) against the NumPy restatement, at
+the shapes where their partition, their lanes per row and their launches have
+edges: one row and column, empty rows and
 columns, rows long enough for a whole warp beside single entries, indices
 over 16 bits, more CTAs than rows, several launches, check intervals that are
 no multiple of its tables. Only the order of the sums differs from the
@@ -36,6 +37,11 @@ def _model(A, seed, lo=0.0, hi=10.0):
                                  q_col_idx=None, q_values=None, q_nnz=0, objective_offset=0.0)
 
 
+def _edge(n_extra):
+    """m + n = 4,096 (the largest float64 LP of the cluster kernel) and past it."""
+    return synthetic.lp_uniform(1300, 2796 + n_extra, 6, seed=12)
+
+
 def _ragged():
     """400 x 900: one full row, one full column, empty rows and columns, single entries."""
     A = sp.random(400, 900, density=0.004, random_state=5, data_rvs=np.random.default_rng(5).standard_normal).tolil()
@@ -51,6 +57,8 @@ MODELS = {
     "one_by_one": lambda: _model(np.array([[1.5]]), 1),
     "fewer_rows_than_ctas": lambda: synthetic.lp_uniform(5, 4000, 2, seed=2),
     "ragged": _ragged,
+    "cluster_largest": lambda: _edge(0),
+    "cluster_past": lambda: _edge(1),
     "wide_indices": lambda: synthetic.lp_uniform(3000, 70001, 3, seed=4),
     "skewed": lambda: synthetic.lp_powerlaw(2001, 4003, 40_000, seed=8),
     "qp": lambda: synthetic.qp_sparse(700, 2001, 5, seed=9),

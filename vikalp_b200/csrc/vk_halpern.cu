@@ -36,6 +36,7 @@
 // tolerance, the iterates move to float64 and the float64 engine finishes
 // (the polish). The answer is always checked in float64.
 #include "vk_engine.cuh"
+#include "vk_halpern_cluster.cuh"
 #include "vk_halpern_resident.cuh"
 #include "vk_power.cuh"
 
@@ -525,7 +526,7 @@ public:
         bool confirmed = false; // mixed: the float32 answer passed the float64 evaluation
         if (mixed_) {
             copy_state<float, double>(s64_, s32_);
-            if (!rs32_ && !g32_) g32_ = capture(s32_);
+            if (!rs32_ && !cl32_ && !g32_) g32_ = capture(s32_);
             // float32 phase. When its own (float32) KKT evaluation reaches the
             // tolerance, the point is evaluated again in float64 with no
             // float64 iteration: accepted there, the solve ends; otherwise the
@@ -547,7 +548,7 @@ public:
                     timed_out = true;
                     break;
                 }
-                advance(s32_, rs32_, g32_);
+                advance(s32_, rs32_ || cl32_, g32_);
                 HalCtl h = hctl_[0];
                 if (h.done) {
                     if (h.status != VK_STATUS_OPTIMAL) break;
@@ -605,13 +606,13 @@ public:
             }
         }
         if (!timed_out && !confirmed) {
-            if (!rs64_ && !g64_) g64_ = capture(s64_);
+            if (!rs64_ && !cl64_ && !g64_) g64_ = capture(s64_);
             for (;;) {
                 if (over_time(started)) {
                     timed_out = true;
                     break;
                 }
-                advance(s64_, rs64_, g64_);
+                advance(s64_, rs64_ || cl64_, g64_);
                 if (hctl_[0].done) break;
             }
         }
@@ -683,7 +684,7 @@ private:
     void advance(HalState<T> &st, bool resident, cudaGraphExec_t g) {
         if (resident) {
             const bool every = sizeof(T) == 4 || o_.verbose >= 2;
-            launch_resident(st, every ? 1 : std::max(1, kRsIterations / chunk_));
+            launch_resident(st, sizeof(T) == 4 ? cl32_ : cl64_, every ? 1 : std::max(1, kRsIterations / chunk_));
             launches_ += 1;
         } else {
             VK_CUDA(cudaGraphLaunch(g, s_));
@@ -708,6 +709,30 @@ private:
         fits_resident<double>(rs64_);
         if (mixed_) fits_resident<float>(rs32_);
         partials_.reset(static_cast<size_t>(kRsMaxGrid) * kCheckSums);
+        // the smallest LPs: one cluster (vk_halpern_cluster.cuh)
+        if (dm_.qp || static_cast<size_t>(dm_.m + dm_.n) * sizeof(float) > kClVectorBytes ||
+            !rs_plan(dm_.a, dm_.at, nullptr, plan_cl_, s_, kClRanks))
+            return;
+        plan_cl_.threads = dm_.nnz <= 8192 ? 256 : kClThreads; // 300 x 800: 2.42 us (512: 2.45); 1,000 x 2,000: 3.70 (256: 3.90)
+        fits_cluster<double>(cl64_);
+        if (mixed_) fits_cluster<float>(cl32_);
+    }
+    template <class T>
+    size_t cluster_layout() const {
+        return ClHalLayout<T>(dm_.m, dm_.n, plan_cl_.cap_a, plan_cl_.cap_t, plan_cl_.rows, plan_cl_.cols).bytes;
+    }
+    template <class T>
+    void fits_cluster(bool &on) {
+        const size_t bytes = cluster_layout<T>();
+        if (static_cast<size_t>(dm_.m + dm_.n) * sizeof(T) > kClVectorBytes || bytes > static_cast<size_t>(kRsSmem)) return;
+        VK_CUDA(cudaFuncSetAttribute(cl_halpern_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRsSmem));
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(kClRanks);
+        cfg.blockDim = dim3(static_cast<unsigned>(plan_cl_.threads));
+        cfg.dynamicSmemBytes = bytes;
+        int clusters = 0;
+        VK_CUDA(cudaOccupancyMaxActiveClusters(&clusters, cl_halpern_kernel<T>, &cfg));
+        on = clusters > 0;
     }
     template <class T>
     void fits_resident(bool &on) {
@@ -728,7 +753,7 @@ private:
             plan_.small ? f(rs_halpern_kernel<T, uint16_t, false>, uint16_t()) : f(rs_halpern_kernel<T, int, false>, int());
     }
     template <class T>
-    void launch_resident(HalState<T> &st, int chunks) {
+    RsHalArgs<T> resident_args(HalState<T> &st, const RsPlan &plan, int chunks) {
         RsHalArgs<T> a{};
         a.ro_a = dm_.a.ro.get();
         a.ci_a = dm_.a.ci.get();
@@ -739,13 +764,13 @@ private:
         a.va = st.ka.get();
         a.vt = st.kat.get();
         a.vq = st.q.get();
-        a.part_a = plan_.part_a.get();
-        a.part_t = plan_.part_t.get();
-        a.cap_a = plan_.cap_a;
-        a.cap_t = plan_.cap_t;
-        a.cap_q = plan_.cap_q;
-        a.rows = plan_.rows;
-        a.cols = plan_.cols;
+        a.part_a = plan.part_a.get();
+        a.part_t = plan.part_t.get();
+        a.cap_a = plan.cap_a;
+        a.cap_t = plan.cap_t;
+        a.cap_q = plan.cap_q;
+        a.rows = plan.rows;
+        a.cols = plan.cols;
         a.x = st.x.get();
         a.x0 = st.x0.get();
         a.xbar = st.xbar.get();
@@ -762,10 +787,21 @@ private:
         a.rs = st.rs.get();
         a.ctl = ctl_.get();
         a.partials = partials_.get();
-        a.counter = plan_.counter.get();
+        a.counter = plan.counter.get();
         a.err = device_error_flag();
         a.chunk = chunk_;
         a.chunks = chunks;
+        return a;
+    }
+    template <class T>
+    void launch_resident(HalState<T> &st, bool cluster, int chunks) {
+        if (cluster) {
+            cl_halpern_kernel<T><<<kClRanks, plan_cl_.threads, cluster_layout<T>(), s_>>>(
+                resident_args(st, plan_cl_, chunks), dm_.m, dm_.n);
+            VK_LAUNCH_CHECK();
+            return;
+        }
+        const RsHalArgs<T> a = resident_args(st, plan_, chunks);
         VK_CUDA(cudaMemsetAsync(plan_.counter.get(), 0, sizeof(unsigned), s_));
         with_kernel<T>([&](auto kernel, auto index) {
             rs_launch(kernel, plan_.grid, plan_.threads, layout<T>(index), s_, a);
@@ -1067,8 +1103,9 @@ private:
     double knorm_ = 0.0, lq_ = 0.0, omega0_ = 1.0, bnorm_ = 0.0, cnorm_ = 0.0;
     cudaGraphExec_t g64_ = nullptr, g32_ = nullptr;
     long long graph_nodes_ = 0, launches_ = 0;
-    RsPlan plan_;
+    RsPlan plan_, plan_cl_;
     bool rs64_ = false, rs32_ = false; // the model is resident in float64 / float32
+    bool cl64_ = false, cl32_ = false; // in one cluster
     DevBuf<double> partials_;
     bool tuned_ = false;
     int col_var_[2] = {-1, -1}, row_var_[2] = {-1, -1}; // tuned pass variants [float64, float32]

@@ -37,7 +37,8 @@ int most_rows(const std::vector<int> &at) {
 }
 } // namespace
 
-bool rs_plan(const CsrPattern32 &a, const CsrPattern32 &at, const CsrPattern32 *q, RsPlan &plan, cudaStream_t s) {
+bool rs_plan(const CsrPattern32 &a, const CsrPattern32 &at, const CsrPattern32 *q, RsPlan &plan, cudaStream_t s,
+             int ctas) {
     if (a.rows == 0 || a.nnz == 0 || forced_variant() >= 0) return false;
     const int64_t stored = 2 * a.nnz + (q ? q->nnz : 0);
     if (stored * static_cast<int64_t>(sizeof(float) + 2) > static_cast<int64_t>(kRsMaxGrid) * kRsSmem) return false;
@@ -47,7 +48,7 @@ bool rs_plan(const CsrPattern32 &a, const CsrPattern32 &at, const CsrPattern32 *
     VK_CUDA(cudaMemcpyAsync(rot.data(), at.ro.get(), rot.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
     if (q) VK_CUDA(cudaMemcpyAsync(roq.data(), q->ro.get(), roq.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
     VK_CUDA(cudaStreamSynchronize(s));
-    plan.grid = rs_grid(a.nnz);
+    plan.grid = ctas > 0 ? ctas : rs_grid(a.nnz);
     plan.threads = rs_threads(a.nnz, plan.grid);
     plan.small = m <= 65536 && n <= 65536;
     // columns are split by their nonzeros in A and Q together

@@ -231,7 +231,9 @@ struct RsPlan {
 
 // Fills `plan` for A, its transpose and (or null) Q; false when the matrices
 // can not fit in any precision, or a kernel variant is pinned.
-bool rs_plan(const CsrPattern32 &a, const CsrPattern32 &at, const CsrPattern32 *q, RsPlan &plan, cudaStream_t s);
+// `ctas`: that many shares (0: rs_grid's).
+bool rs_plan(const CsrPattern32 &a, const CsrPattern32 &at, const CsrPattern32 *q, RsPlan &plan, cudaStream_t s,
+             int ctas = 0);
 
 // CTAs (at most one per SM) and threads for `nnz` nonzeros. Timed per
 // iteration (float64 Halpern, 37 / 74 / 148 CTAs x 256 / 512 / 768 / 1024
