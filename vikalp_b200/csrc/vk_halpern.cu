@@ -709,11 +709,11 @@ private:
         fits_resident<double>(rs64_);
         if (mixed_) fits_resident<float>(rs32_);
         partials_.reset(static_cast<size_t>(kRsMaxGrid) * kCheckSums);
-        // the smallest LPs: one cluster (vk_halpern_cluster.cuh)
+        // the smallest LPs: one cluster (vk_cluster.cuh)
         if (dm_.qp || static_cast<size_t>(dm_.m + dm_.n) * sizeof(float) > kClVectorBytes ||
             !rs_plan(dm_.a, dm_.at, nullptr, plan_cl_, s_, kClRanks))
             return;
-        plan_cl_.threads = dm_.nnz <= 8192 ? 256 : kClThreads; // 300 x 800: 2.42 us (512: 2.45); 1,000 x 2,000: 3.70 (256: 3.90)
+        plan_cl_.threads = cl_threads(dm_.nnz);
         fits_cluster<double>(cl64_);
         if (mixed_) fits_cluster<float>(cl32_);
     }
@@ -723,16 +723,8 @@ private:
     }
     template <class T>
     void fits_cluster(bool &on) {
-        const size_t bytes = cluster_layout<T>();
-        if (static_cast<size_t>(dm_.m + dm_.n) * sizeof(T) > kClVectorBytes || bytes > static_cast<size_t>(kRsSmem)) return;
-        VK_CUDA(cudaFuncSetAttribute(cl_halpern_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRsSmem));
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(kClRanks);
-        cfg.blockDim = dim3(static_cast<unsigned>(plan_cl_.threads));
-        cfg.dynamicSmemBytes = bytes;
-        int clusters = 0;
-        VK_CUDA(cudaOccupancyMaxActiveClusters(&clusters, cl_halpern_kernel<T>, &cfg));
-        on = clusters > 0;
+        if (static_cast<size_t>(dm_.m + dm_.n) * sizeof(T) > kClVectorBytes) return;
+        on = cl_fits(cl_halpern_kernel<T>, plan_cl_.threads, cluster_layout<T>());
     }
     template <class T>
     void fits_resident(bool &on) {

@@ -30,6 +30,7 @@
 // Chunks of iterations are captured in a CUDA graph; the host only polls a
 // done flag between chunks.
 #include "vk_engine.cuh"
+#include "vk_reference_cluster.cuh"
 #include "vk_reference_resident.cuh"
 
 #include <algorithm>
@@ -536,10 +537,21 @@ private:
     // (vk_resident.cuh); pinned variants keep the passes.
     void plan_resident() {
         const char *pinned = std::getenv("VIKALP_B200_PASS_VARIANTS");
-        if (exact_ || dm_.qp || (pinned && *pinned) || !rs_plan(dm_.a, dm_.at, nullptr, plan_, s_)) return;
+        if (exact_ || dm_.qp || (pinned && *pinned)) return;
+        // the smallest: one cluster (vk_cluster.cuh)
+        if (static_cast<size_t>(dm_.m + dm_.n) * sizeof(double) <= kClVectorBytes &&
+            rs_plan(dm_.a, dm_.at, nullptr, plan_, s_, kClRanks)) {
+            plan_.threads = cl_threads(dm_.nnz);
+            resident_ = cluster_ = cl_fits(cl_reference_kernel, plan_.threads, cluster_layout());
+            if (cluster_) return;
+        }
+        if (!rs_plan(dm_.a, dm_.at, nullptr, plan_, s_)) return;
         resident_ = plan_.small ? rs_fits(rs_reference_kernel<uint16_t>, plan_.grid, plan_.threads, layout<uint16_t>())
                                 : rs_fits(rs_reference_kernel<int>, plan_.grid, plan_.threads, layout<int>());
         norms_.reset(8);
+    }
+    size_t cluster_layout() const {
+        return ClRefLayout(dm_.m, dm_.n, plan_.cap_a, plan_.cap_t, plan_.rows, plan_.cols).bytes;
     }
     template <class I>
     size_t layout() const {
@@ -574,6 +586,11 @@ private:
         a.counter = plan_.counter.get();
         a.err = device_error_flag();
         a.iterations = kRsIterations;
+        if (cluster_) {
+            cl_reference_kernel<<<kClRanks, plan_.threads, cluster_layout(), s_>>>(a, dm_.m, dm_.n);
+            VK_LAUNCH_CHECK();
+            return;
+        }
         VK_CUDA(cudaMemsetAsync(plan_.counter.get(), 0, sizeof(unsigned), s_));
         VK_CUDA(cudaMemsetAsync(norms_.get(), 0, norms_.bytes(), s_));
         if (plan_.small)
@@ -801,7 +818,7 @@ private:
     long long graph_nodes_ = 0;
     cudaGraphExec_t graph_exec_ = nullptr;
     RsPlan plan_;
-    bool resident_ = false;
+    bool resident_ = false, cluster_ = false; // iterations run in shared memory; in one cluster
     DevBuf<double> norms_;
 };
 
