@@ -251,7 +251,7 @@ __global__ void ref_control_kernel(RefCtl *ctl) {
     pdl_wait();
     RefCtl c = *ctl;
     if (c.done) return;
-    ref_decide(c);
+    ref_decide(c, ref_policy_iter(c.iter));
     *ctl = c;
 }
 

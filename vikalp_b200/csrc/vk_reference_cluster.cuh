@@ -1,8 +1,10 @@
 // The reference scheme on an LP in one thread-block cluster (vk_cluster.cuh):
 // the iterations of vk_reference_resident.cuh, control steps included,
-// `iterations` of them in one launch. Microseconds per iteration against the
-// resident kernel: 5 x 8 LP 3.07 (5.56), 300 x 800 3.62 (6.19), 1,000 x 2,000 with
-// 16,000 nonzeros 4.63 (6.36), 1,300 x 2,700 with 32,400 5.95 (6.82).
+// `iterations` of them in one launch. Microseconds per iteration: 5 x 8 LP 2.36,
+// 300 x 800 2.92, 1,000 x 2,000 with 16,000 nonzeros 4.12, 1,300 x 2,700 with
+// 32,400 5.35 (with the division and the shuffled maxima that the control step
+// had before, 3.07, 3.62, 4.63 and 5.95 against 5.56, 6.19, 6.36 and 6.82 of the
+// resident kernel, which has since gained a microsecond too).
 #pragma once
 
 #include "vk_cluster.cuh"
@@ -17,15 +19,15 @@ using ClRefLayout = ClLayout<double, 6, 4>;
 // slot in every rank's copy.
 __device__ __forceinline__ void cl_put_max(double v, double (*slots)[kClThreads / 32], int rank) {
     const int lane = threadIdx.x & 31;
-    v = warp_max_nonneg(v);
+    v = rs_warp_max(v);
     if (lane < kClRanks) cl_store(cl_map(smem_u32(&slots[rank][threadIdx.x >> 5]), lane), v);
 }
-// The maximum over all slots, in every lane of the calling warp.
-__device__ __forceinline__ double cl_max(const double (*slots)[kClThreads / 32]) {
-    const int warps = static_cast<int>(blockDim.x) >> 5;
+// The lane's part of the maximum over all slots.
+__device__ __forceinline__ double cl_part_max(const double (*slots)[kClThreads / 32]) {
     double v = 0.0;
-    for (int i = threadIdx.x & 31; i < kClRanks * warps; i += 32) v = smax(v, slots[i / warps][i % warps]);
-    return warp_max_nonneg(v);
+#pragma unroll
+    for (int i = 0; i < kClRanks * (kClThreads / 32); i += 32) v = smax(v, (&slots[0][0])[i + (threadIdx.x & 31)]);
+    return v;
 }
 
 __global__ void __cluster_dims__(kClRanks, 1, 1) __launch_bounds__(kClThreads, 1)
@@ -62,8 +64,11 @@ __global__ void __cluster_dims__(kClRanks, 1, 1) __launch_bounds__(kClThreads, 1
         ru[i] = A.ru[r0 + i];
     }
     for (int i = tid; i < m; i += nt) yf[i] = A.y[i];
+    for (int i = tid; i < kClRanks * (kClThreads / 32); i += nt) // with fewer warps, the rest stay 0
+        (&stat[0][0])[i] = (&prim[0][0][0])[i] = (&prim[1][0][0])[i] = 0.0;
     cl_sync(); // every rank has started (remote stores may reach it) and is loaded
     const long long start = c.iter, end = start + A.iterations;
+    RefPhase phase(start);
     long long *const cycles = rank == 0 && tid == 0 ? A.cycles : nullptr;
     long long mark = cycles ? clock64() : 0;
     const auto lap = [&](int q) {
@@ -78,10 +83,10 @@ __global__ void __cluster_dims__(kClRanks, 1, 1) __launch_bounds__(kClThreads, 1
     struct RowIn {
         double y, kx, lo, hi;
     };
-    for (long long k = start;; ++k) {
+    for (long long k = start;; ++k, phase.next()) {
         // K'y_k, the stationarity of iteration k-1, and the primal step of
         // iteration k unless the control step may still change tau
-        const bool policy = ref_policy_iter(k);
+        const bool policy = phase.policy(k);
         const double tau = c.tau;
         double top = 0.0;
         const auto column = [&](int j) { return ColIn{x[j], cc[j], l[j], u[j]}; };
@@ -103,13 +108,17 @@ __global__ void __cluster_dims__(kClRanks, 1, 1) __launch_bounds__(kClThreads, 1
         lap(0);
         // control: every rank from the same numbers
         if (tid < 32) {
-            const double rp = cl_max(prim[(k + 1) & 1]), rd = cl_max(stat);
+            // (the decision takes the larger of the two norms; the launch's last
+            // step keeps the primal one, its column pass will be repeated)
+            double v = cl_part_max(prim[(k + 1) & 1]);
+            if (k < end) v = smax(v, cl_part_max(stat));
+            v = rs_warp_max(v);
             if (tid == 0) {
-                if (k > start) c.rp = rp;
-                if (k < end) {
-                    c.rd = rd;
-                    ref_decide(c);
-                }
+                if (k == start)
+                    c.rd = v;
+                else
+                    c.rp = v;
+                if (k < end) ref_decide(c, policy);
             }
         }
         __syncthreads();

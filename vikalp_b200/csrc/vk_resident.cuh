@@ -158,6 +158,15 @@ __device__ __forceinline__ bool rs_block(bool ok, int *err) {
     return __syncthreads_or(!ok) == 0;
 }
 
+// The warp's maximum of v >= 0 (no NaN): such doubles order as their bits do, so
+// that two integer reductions do for five steps of shuffles and comparisons.
+__device__ __forceinline__ double rs_warp_max(double v) {
+    const unsigned hi = static_cast<unsigned>(__double2hiint(v)), lo = static_cast<unsigned>(__double2loint(v));
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+    return __hiloint2double(static_cast<int>(mh), static_cast<int>(ml));
+}
+
 // Grid barrier over the gridDim.x CTAs of a cooperative launch; `counter` is
 // zero at the launch. All writes before it are visible after it.
 struct RsBarrier {
@@ -173,12 +182,12 @@ struct RsBarrier {
     // The same, and *slot becomes the largest of itself and every thread's v
     // (non-negative; NaN ignored). `warps`: 32 doubles of shared memory.
     __device__ __forceinline__ bool sync_max(double v, double *warps, double *slot) {
-        v = warp_max_nonneg(v);
+        v = rs_warp_max(v);
         if ((threadIdx.x & 31) == 0) warps[threadIdx.x >> 5] = v;
         __syncthreads();
-        if (threadIdx.x == 0) {
-            for (unsigned w = 1; w < blockDim.x / 32; ++w) v = smax(v, warps[w]);
-            atomic_max_nonneg(slot, v);
+        if (threadIdx.x < 32) {
+            v = rs_warp_max(threadIdx.x < blockDim.x / 32 ? warps[threadIdx.x] : 0.0);
+            if (threadIdx.x == 0) atomic_max_nonneg(slot, v);
         }
         return arrive_and_wait();
     }
