@@ -171,7 +171,8 @@ void vk_pdhg_destroy(vk_pdhg *h);
  * stream. For measurement only (no counterpart in the reference, whose
  * backend calls are timed by nothing). VK_ALGO_REFERENCE handles report
  * three kinds: the column pass, the control (+ primal) kernels and the row
- * pass; other schemes return VK_ERR_UNSUPPORTED. */
+ * pass (a model that iterates inside one kernel: its device time, divided by
+ * the cycles that one block counted in the three parts); other schemes return VK_ERR_UNSUPPORTED. */
 typedef struct {
     int32_t count;             /* kernel kinds reported (<= 8)                  */
     char name[8][48];

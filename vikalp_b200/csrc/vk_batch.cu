@@ -2251,9 +2251,9 @@ void batch_solve_together(const vk_problem &shared, int node_count, const double
     validate_batch(probs, count, o);
     const auto t0 = std::chrono::steady_clock::now();
     {
-        // both set-ups first (they allocate and free device memory, which
-        // synchronises the device), then both iteration loops at once, each
-        // engine on its own stream from its own host thread
+        // both set-ups first (their host round trips would queue behind the
+        // other's passes), then both iteration loops at once, each engine on its
+        // own stream from its own host thread
         SharedEngine nodes(shared, node_count, o);
         BatchEngine lps(probs, count, o);
         if (o.verbose > 0)

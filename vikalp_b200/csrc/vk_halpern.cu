@@ -24,7 +24,9 @@
 // previous check, or k >= 0.2 * total iterations; PrimalWeightRule,
 // vk_engine.cuh), restarting at (x^, y^) and updating the primal weight omega
 // by the smoothed (theta = 0.2) log-ratio of the moves of the restart points.
-// The chunk of check_every iterations is one CUDA graph.
+// The chunk of check_every iterations is one CUDA graph. Models whose matrices
+// fit the shared memory of the GPU, or of one cluster, run the same steps in one
+// kernel instead (vk_halpern_resident.cuh, vk_halpern_cluster.cuh).
 //
 // Setup: 10 Ruiz infinity-norm passes then one Pock-Chambolle (alpha = 1)
 // pass give R and D; eta = 0.99 / sigma_max(K) with sigma_max from power

@@ -28,7 +28,9 @@
 //     every-50th, pdhg.cpp:133), so the separate primal kernel runs once per
 //     50 iterations.
 // Chunks of iterations are captured in a CUDA graph; the host only polls a
-// done flag between chunks.
+// done flag between chunks. FAST-order LPs whose matrices fit the shared memory
+// of the GPU, or of one cluster, run the same steps in one kernel instead
+// (vk_reference_resident.cuh, vk_reference_cluster.cuh).
 #include "vk_engine.cuh"
 #include "vk_reference_cluster.cuh"
 #include "vk_reference_resident.cuh"
