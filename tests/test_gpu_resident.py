@@ -1,10 +1,10 @@
 """Solves whose model iterates in the shared memory of one cluster or of the GPU
 (vk_halpern_cluster.cuh, vk_resident.cuh) against the NumPy restatement, at
 the shapes where their partition, their lanes per row and their launches have
-edges: one row and column, empty rows and
-columns, rows long enough for a whole warp beside single entries, indices
-over 16 bits, more CTAs than rows, several launches, check intervals that are
-no multiple of its tables. Only the order of the sums differs from the
+edges: one row and column, empty rows and columns, rows long enough for a whole
+warp beside single entries, indices over 16 bits and over the packed 19, more
+CTAs than rows, several launches, check intervals that are no multiple of its
+tables. Only the order of the sums differs from the
 restatement: 1e-8 relative after a few hundred iterations, as for the passes."""
 
 import types
@@ -53,6 +53,13 @@ def _ragged():
     return _model(A.tocsr(), 7)
 
 
+def _wide(n):
+    """2,000 rows, entries in every 13th column and in the first and last of n, the rest empty."""
+    rng = np.random.default_rng(14)
+    cols = np.r_[0, np.arange(1, n - 1, 13), n - 1]
+    return _model(sp.csr_matrix((rng.standard_normal(len(cols)), (rng.integers(0, 2000, len(cols)), cols)), (2000, n)), 15)
+
+
 MODELS = {
     "one_by_one": lambda: _model(np.array([[1.5]]), 1),
     "fewer_rows_than_ctas": lambda: synthetic.lp_uniform(5, 4000, 2, seed=2),
@@ -61,6 +68,11 @@ MODELS = {
     "cluster_past": lambda: _edge(1),
     "wide_indices": lambda: synthetic.lp_uniform(3000, 70001, 3, seed=4),
     "skewed": lambda: synthetic.lp_powerlaw(2001, 4003, 40_000, seed=8),
+    # 19 bits hold the columns of a packed index: the last LP that they do, the
+    # first that they don't, and shares that only fit with 16-bit indices
+    "widest_packed": lambda: _wide(1 << 19),
+    "past_packed": lambda: _wide((1 << 19) + 1),
+    "long_rows_16_bit": lambda: synthetic.lp_uniform(4000, 8000, 138, seed=13),
     "qp": lambda: synthetic.qp_sparse(700, 2001, 5, seed=9),
 }
 

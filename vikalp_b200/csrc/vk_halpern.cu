@@ -703,13 +703,14 @@ private:
     }
 
     // A model whose matrices fit the GPU's shared memory iterates there
-    // (vk_resident.cuh): 10.3 us an iteration against 23.7 for the passes at
-    // 600,000 nonzeros, 16.1 against 37.5 at 720,000 (float64; past about
-    // 800,000 they no longer fit), 17.5 against 26.4 at 940,000 (float32).
+    // (vk_resident.cuh): 9.5 us an iteration against 23.7 for the passes at
+    // 600,000 nonzeros (float64), and, with the gathers still in row order, 16.1
+    // against 37.5 at 720,000 (past about 800,000 they no longer fit), 17.5
+    // against 26.4 at 940,000 (float32).
     void plan_resident() {
         if (!rs_plan(dm_.a, dm_.at, dm_.qp ? &dm_.q : nullptr, plan_, s_)) return;
-        fits_resident<double>(rs64_);
-        if (mixed_) fits_resident<float>(rs32_);
+        fits_resident<double>(rs64_, packed64_);
+        if (mixed_) fits_resident<float>(rs32_, packed32_);
         partials_.reset(static_cast<size_t>(kRsMaxGrid) * kCheckSums);
         // the smallest LPs: one cluster (vk_cluster.cuh)
         if (dm_.qp || static_cast<size_t>(dm_.m + dm_.n) * sizeof(float) > kClVectorBytes ||
@@ -729,10 +730,13 @@ private:
         on = cl_fits(cl_halpern_kernel<T>, plan_cl_.threads, cluster_layout<T>());
     }
     template <class T>
-    void fits_resident(bool &on) {
-        with_kernel<T>([&](auto kernel, auto index) {
-            on = rs_fits(kernel, plan_.grid, plan_.threads, layout<T>(index));
-        });
+    void fits_resident(bool &on, bool &packed) {
+        for (packed = plan_.packed;; packed = false) {
+            with_kernel<T>(packed, [&](auto kernel, auto index) {
+                on = rs_fits(kernel, plan_.grid, plan_.threads, layout<T>(index));
+            });
+            if (on || !packed) return;
+        }
     }
     template <class T, class I>
     size_t layout(I) const {
@@ -740,21 +744,20 @@ private:
     }
     // f(kernel, a value of its index type)
     template <class T, class F>
-    void with_kernel(F &&f) {
-        if (dm_.qp)
-            plan_.small ? f(rs_halpern_kernel<T, uint16_t, true>, uint16_t()) : f(rs_halpern_kernel<T, int, true>, int());
-        else
-            plan_.small ? f(rs_halpern_kernel<T, uint16_t, false>, uint16_t()) : f(rs_halpern_kernel<T, int, false>, int());
+    void with_kernel(bool packed, F &&f) {
+        rs_with_index(plan_, packed, [&](auto i) {
+            dm_.qp ? f(rs_halpern_kernel<T, decltype(i), true>, i) : f(rs_halpern_kernel<T, decltype(i), false>, i);
+        });
     }
     template <class T>
-    RsHalArgs<T> resident_args(HalState<T> &st, const RsPlan &plan, int chunks) {
+    RsHalArgs<T> resident_args(HalState<T> &st, const RsPlan &plan, bool packed, int chunks) {
         RsHalArgs<T> a{};
         a.ro_a = dm_.a.ro.get();
-        a.ci_a = dm_.a.ci.get();
+        a.ci_a = plan.index(plan.words_a, dm_.a, packed);
         a.ro_t = dm_.at.ro.get();
-        a.ci_t = dm_.at.ci.get();
+        a.ci_t = plan.index(plan.words_t, dm_.at, packed);
         a.ro_q = dm_.q.ro.get();
-        a.ci_q = dm_.q.ci.get();
+        a.ci_q = plan.index(plan.words_q, dm_.q, packed);
         a.va = st.ka.get();
         a.vt = st.kat.get();
         a.vq = st.q.get();
@@ -791,13 +794,14 @@ private:
     void launch_resident(HalState<T> &st, bool cluster, int chunks) {
         if (cluster) {
             cl_halpern_kernel<T><<<kClRanks, plan_cl_.threads, cluster_layout<T>(), s_>>>(
-                resident_args(st, plan_cl_, chunks), dm_.m, dm_.n);
+                resident_args(st, plan_cl_, false, chunks), dm_.m, dm_.n);
             VK_LAUNCH_CHECK();
             return;
         }
-        const RsHalArgs<T> a = resident_args(st, plan_, chunks);
+        const bool packed = sizeof(T) == 4 ? packed32_ : packed64_;
+        const RsHalArgs<T> a = resident_args(st, plan_, packed, chunks);
         VK_CUDA(cudaMemsetAsync(plan_.counter.get(), 0, sizeof(unsigned), s_));
-        with_kernel<T>([&](auto kernel, auto index) {
+        with_kernel<T>(packed, [&](auto kernel, auto index) {
             rs_launch(kernel, plan_.grid, plan_.threads, layout<T>(index), s_, a);
         });
     }
@@ -1099,6 +1103,7 @@ private:
     long long graph_nodes_ = 0, launches_ = 0;
     RsPlan plan_, plan_cl_;
     bool rs64_ = false, rs32_ = false; // the model is resident in float64 / float32
+    bool packed64_ = false, packed32_ = false; // with RsPacked indices
     bool cl64_ = false, cl32_ = false; // in one cluster
     DevBuf<double> partials_;
     bool tuned_ = false;

@@ -548,8 +548,13 @@ private:
             if (cluster_) return;
         }
         if (!rs_plan(dm_.a, dm_.at, nullptr, plan_, s_)) return;
-        resident_ = plan_.small ? rs_fits(rs_reference_kernel<uint16_t>, plan_.grid, plan_.threads, layout<uint16_t>())
-                                : rs_fits(rs_reference_kernel<int>, plan_.grid, plan_.threads, layout<int>());
+        for (;; plan_.packed = false) {
+            rs_with_index(plan_, plan_.packed, [&](auto i) {
+                using I = decltype(i);
+                resident_ = rs_fits(rs_reference_kernel<I>, plan_.grid, plan_.threads, layout<I>());
+            });
+            if (resident_ || !plan_.packed) break;
+        }
         norms_.reset(8);
     }
     size_t cluster_layout() const {
@@ -563,9 +568,9 @@ private:
         RsRefArgs a{};
         a.cycles = cycles;
         a.ro_a = dm_.a.ro.get();
-        a.ci_a = dm_.a.ci.get();
+        a.ci_a = plan_.index(plan_.words_a, dm_.a, plan_.packed);
         a.ro_t = dm_.at.ro.get();
-        a.ci_t = dm_.at.ci.get();
+        a.ci_t = plan_.index(plan_.words_t, dm_.at, plan_.packed);
         a.va = ka_.get();
         a.vt = kat_.get();
         a.part_a = plan_.part_a.get();
@@ -595,10 +600,10 @@ private:
         }
         VK_CUDA(cudaMemsetAsync(plan_.counter.get(), 0, sizeof(unsigned), s_));
         VK_CUDA(cudaMemsetAsync(norms_.get(), 0, norms_.bytes(), s_));
-        if (plan_.small)
-            rs_launch(rs_reference_kernel<uint16_t>, plan_.grid, plan_.threads, layout<uint16_t>(), s_, a);
-        else
-            rs_launch(rs_reference_kernel<int>, plan_.grid, plan_.threads, layout<int>(), s_, a);
+        rs_with_index(plan_, plan_.packed, [&](auto i) {
+            using I = decltype(i);
+            rs_launch(rs_reference_kernel<I>, plan_.grid, plan_.threads, layout<I>(), s_, a);
+        });
     }
 
     void iteration(int k) { iteration_parts(k, nullptr); }

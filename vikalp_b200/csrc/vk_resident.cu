@@ -35,6 +35,43 @@ int most_rows(const std::vector<int> &at) {
     for (size_t b = 0; b + 1 < at.size(); ++b) most = std::max(most, at[b + 1] - at[b]);
     return most;
 }
+constexpr int kRsPlaces = 1 << RsPacked::kPlaceBits;
+
+// out: the RsPacked words of every share, in column order (places ascending
+// within a column). One CTA sorts a share in shared memory (bitonic): about 25 us
+// for 600,000 nonzeros, once per handle; sorted again by every launch it had cost
+// the solves of less than 64 iterations more than the order gave them.
+__global__ void __launch_bounds__(1024) rs_pack_kernel(const int *__restrict__ ro, const int *__restrict__ ci,
+                                                       const int *__restrict__ part, int count, int *__restrict__ out) {
+    extern __shared__ uint32_t key[]; // count: a power of two, at least the share
+    const int k0 = ro[part[blockIdx.x]], nnz = ro[part[blockIdx.x + 1]] - k0;
+    for (int k = threadIdx.x; k < count; k += blockDim.x)
+        key[k] = k < nnz ? static_cast<uint32_t>(ci[k0 + k]) << RsPacked::kPlaceBits | static_cast<uint32_t>(k)
+                         : 0xffffffffu; // not below any word
+    for (int size = 2; size <= count; size <<= 1)
+        for (int gap = size >> 1; gap > 0; gap >>= 1) {
+            __syncthreads();
+            for (int t = threadIdx.x; t < count / 2; t += blockDim.x) {
+                const int a = 2 * t - (t & (gap - 1)), b = a + gap;
+                const uint32_t ka = key[a], kb = key[b];
+                if ((ka > kb) == ((a & size) == 0)) {
+                    key[a] = kb;
+                    key[b] = ka;
+                }
+            }
+        }
+    __syncthreads();
+    for (int k = threadIdx.x; k < nnz; k += blockDim.x) out[k0 + k] = static_cast<int>(key[k]);
+}
+
+void pack(const CsrPattern32 &p, const DevBuf<int> &part, int grid, int cap, DevBuf<int> &out, cudaStream_t s) {
+    out.reset(std::max<int64_t>(p.nnz, 1));
+    int count = 2;
+    while (count < cap) count *= 2;
+    rs_pack_kernel<<<grid, std::min(1024, std::max(32, count / 2)), count * sizeof(uint32_t), s>>>(
+        p.ro.get(), p.ci.get(), part.get(), count, out.get());
+    VK_LAUNCH_CHECK();
+}
 } // namespace
 
 bool rs_plan(const CsrPattern32 &a, const CsrPattern32 &at, const CsrPattern32 *q, RsPlan &plan, cudaStream_t s,
@@ -65,6 +102,15 @@ bool rs_plan(const CsrPattern32 &a, const CsrPattern32 &at, const CsrPattern32 *
     plan.counter.reset(1);
     VK_CUDA(cudaMemcpyAsync(plan.part_a.get(), pa.data(), plan.part_a.bytes(), cudaMemcpyHostToDevice, s));
     VK_CUDA(cudaMemcpyAsync(plan.part_t.get(), pt.data(), plan.part_t.bytes(), cudaMemcpyHostToDevice, s));
+    // column order: a plan for the whole GPU whose columns and shares fit the bits
+    constexpr int kCols = 1 << RsPacked::kColBits;
+    const int most = std::max({plan.cap_a, plan.cap_t, plan.cap_q});
+    plan.packed = ctas == 0 && m <= kCols && n <= kCols && most <= kRsPlaces;
+    if (plan.packed) {
+        pack(a, plan.part_a, plan.grid, plan.cap_a, plan.words_a, s);
+        pack(at, plan.part_t, plan.grid, plan.cap_t, plan.words_t, s);
+        if (q) pack(*q, plan.part_t, plan.grid, plan.cap_q, plan.words_q, s);
+    }
     VK_CUDA(cudaStreamSynchronize(s)); // the boundaries live on this stack frame
     return true;
 }

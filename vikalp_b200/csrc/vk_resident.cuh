@@ -9,8 +9,8 @@
 // through L2: a pass gathers, multiplies, sums its rows and writes its own
 // slice of the other vector, and one grid barrier orders the passes. The
 // gathers are taken nonzero by nonzero (every thread the same number in
-// flight, whatever the row lengths), the products staged in shared memory and
-// the row sums taken from there.
+// flight, whatever the row lengths) and in column order (RsPacked), the products
+// staged in shared memory in row order and the row sums taken from there.
 //
 // The grid barrier spins on a counter in L2 (2,550 cycles with 148 CTAs;
 // flags polled by every CTA and a two-level tree took 4,300-7,300, and packets
@@ -21,6 +21,8 @@
 #pragma once
 
 #include "vk_csr.cuh"
+
+#include <type_traits>
 
 namespace vk {
 
@@ -45,13 +47,43 @@ struct RsSide {
     bool longs; // some row goes to a whole warp
 };
 
+// The index of a nonzero that is gathered in column order: its column, and its
+// place in the share (row order), where its product goes. A warp's gathers then
+// share cache lines, and an L1 looks up one line a cycle (a share of 4,000
+// nonzeros has 4,000 lookups in row order and 2,300-3,000 lines); the products
+// land in the same places, so that the sums stay what they were. Measured, per
+// float64 Halpern iteration: 4,000 x 8,000 LP with 240,000 nonzeros 9.02 -> 6.13 us,
+// 50,000 x 100,000 with 600,000 10.44 -> 9.52, QP 40,000 x 100,000 15.75 -> 13.71, a
+// power law of 528,000 12.01 -> 9.80, 2,000 x 5,000 with 40,000 5.14 -> 5.12 (float32,
+// with the float64 finish: 10.57 -> 6.31, 11.06 -> 8.85, 13.00 -> 10.71, 13.26 -> 9.40).
+// Hence every plan whose columns and shares its bits can hold is packed, unless
+// only 16-bit indices leave room for the matrices.
+struct RsPacked {
+    static constexpr int kPlaceBits = 13, kColBits = 32 - kPlaceBits;
+    uint32_t w;
+};
+template <class I>
+__device__ __forceinline__ int rs_col(I i) { return static_cast<int>(i); }
+__device__ __forceinline__ int rs_col(RsPacked i) { return static_cast<int>(i.w >> RsPacked::kPlaceBits); }
+template <class I>
+__device__ __forceinline__ int rs_place(I, int k) { return k; }
+__device__ __forceinline__ int rs_place(RsPacked i, int) {
+    return static_cast<int>(i.w & ((1u << RsPacked::kPlaceBits) - 1u));
+}
+
 template <class T, class I>
 __device__ RsSide<T, I> rs_load(const int *__restrict__ ro, const int *__restrict__ ci, const T *__restrict__ val,
                                 int r0, int r1, T *v, I *idx, int *sro) {
     const int k0 = ro[r0], nnz = ro[r1] - k0, rows = r1 - r0;
     for (int k = threadIdx.x; k < nnz; k += blockDim.x) {
-        v[k] = __ldg(val + k0 + k);
-        idx[k] = static_cast<I>(__ldg(ci + k0 + k));
+        const int w = __ldg(ci + k0 + k);
+        if constexpr (std::is_same_v<I, RsPacked>) { // ci: the plan's packed words
+            idx[k] = RsPacked{static_cast<uint32_t>(w)};
+            v[k] = __ldg(val + k0 + rs_place(idx[k], k));
+        } else {
+            idx[k] = static_cast<I>(w);
+            v[k] = __ldg(val + k0 + k);
+        }
     }
     // lanes per row: every thread busy in one round, at most about one per nonzero
     int L = 1;
@@ -72,20 +104,29 @@ __device__ __forceinline__ void rs_products(const RsSide<T, I> &s, const T *x, A
     int k = threadIdx.x;
     for (; k + (kRsGather - 1) * nt < s.nnz; k += kRsGather * nt) {
         T g[kRsGather];
+        I i[kRsGather];
 #pragma unroll
-        for (int u = 0; u < kRsGather; ++u) g[u] = __ldcg(x + s.idx[k + u * nt]);
+        for (int u = 0; u < kRsGather; ++u) {
+            i[u] = s.idx[k + u * nt];
+            g[u] = __ldcg(x + rs_col(i[u]));
+        }
 #pragma unroll
         for (int u = 0; u < kRsGather; ++u)
-            prod[k + u * nt] = static_cast<A>(s.v[k + u * nt]) * static_cast<A>(g[u]);
+            prod[rs_place(i[u], k + u * nt)] = static_cast<A>(s.v[k + u * nt]) * static_cast<A>(g[u]);
     }
     if (k < s.nnz) { // fewer than kRsGather left
         T g[kRsGather];
+        I i[kRsGather];
 #pragma unroll
         for (int u = 0; u < kRsGather; ++u)
-            if (k + u * nt < s.nnz) g[u] = __ldcg(x + s.idx[k + u * nt]);
+            if (k + u * nt < s.nnz) {
+                i[u] = s.idx[k + u * nt];
+                g[u] = __ldcg(x + rs_col(i[u]));
+            }
 #pragma unroll
         for (int u = 0; u < kRsGather; ++u)
-            if (k + u * nt < s.nnz) prod[k + u * nt] = static_cast<A>(s.v[k + u * nt]) * static_cast<A>(g[u]);
+            if (k + u * nt < s.nnz)
+                prod[rs_place(i[u], k + u * nt)] = static_cast<A>(s.v[k + u * nt]) * static_cast<A>(g[u]);
     }
 }
 
@@ -231,11 +272,17 @@ __device__ __forceinline__ bool rs_sum(double (&v)[NR], double *partials, double
 
 // The launch of a model: its shape, the largest shares, the shares' boundaries.
 struct RsPlan {
-    bool small = false; // 16-bit indices
+    bool small = false;  // 16-bit indices
+    bool packed = false; // gathers in column order (RsPacked)
     int grid = 0, threads = 0;
     int cap_a = 0, cap_t = 0, cap_q = 0, rows = 0, cols = 0;
     DevBuf<int> part_a, part_t;
     DevBuf<unsigned> counter; // of the grid barrier
+    DevBuf<int> words_a, words_t, words_q; // packed: RsPacked, share by share
+    // the index array of a launch
+    const int *index(const DevBuf<int> &words, const CsrPattern32 &p, bool use_packed) const {
+        return use_packed ? words.get() : p.ci.get();
+    }
 };
 
 // Fills `plan` for A, its transpose and (or null) Q; false when the matrices
@@ -250,6 +297,16 @@ bool rs_plan(const CsrPattern32 &a, const CsrPattern32 &at, const CsrPattern32 *
 // nonzeros 5.2 us with 148 x 256 (37 x 256: 6.5, 148 x 1024: 5.5), 120,000
 // nonzeros 6.0 us with 148 x 512 (256: 6.4, 1024: 6.5), 600,000 nonzeros 10.3
 // us with 148 x 768 (256: 12.2, 1024: 10.9).
+// f(a value of the index type of a launch): the plan's, or without its packing.
+template <class F>
+void rs_with_index(const RsPlan &plan, bool packed, F &&f) {
+    if (packed)
+        f(RsPacked());
+    else if (plan.small)
+        f(uint16_t());
+    else
+        f(int());
+}
 int rs_grid(int64_t nnz);
 int rs_threads(int64_t nnz, int grid);
 
