@@ -29,7 +29,9 @@ namespace vk {
 constexpr int kRsThreads = 768;     // threads of a CTA, at most
 constexpr int kRsSmem = 220 * 1024; // dynamic shared memory of a CTA (227 KB less the static part)
 constexpr int kRsRowCost = 4;       // partition: a row costs this many nonzeros
-constexpr int kRsGather = 4;        // gathers in flight per thread
+// gathers in flight per thread: 50,000 x 100,000 LP 9.5 us an iteration with 2 or 4, 10.4 with 6
+// or 8; QP 40,000 x 100,000 13.2 / 13.6 / 14.8 / 15.5; 4,000 x 8,000 6.4 / 6.1 / 6.5 / 7.0
+constexpr int kRsGather = 4;
 constexpr int kRsWarpRow = 32;      // a row of more than this many products per lane goes to a whole warp
 constexpr int kRsMaxGrid = 160;
 constexpr int kRsIterations = 1024; // iterations in one launch, about
