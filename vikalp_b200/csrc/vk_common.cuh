@@ -245,8 +245,10 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
 // Programmatic dependent launch. A kernel launched by launch_after starts while
 // the kernel before it on the stream drains (its CTAs take slots as they come
 // free) and calls pdl_wait before it touches anything; that returns once the
-// kernel before it has completed, so nothing else changes for either. Saves the
-// launch gap between the passes of an iteration.
+// kernel before it has completed and its writes are visible to ordinary loads.
+// Its grid is alive while those writes happen, so what the kernel before writes
+// is never read by __ldg (ld.global.nc: memory that is read-only for the life of
+// the grid). Saves the launch gap between the passes of an iteration.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void pdl_wait() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -128,10 +128,20 @@ __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, 
 __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
 
+// The gathered vectors. A FAST pass may be resident while the pass before it still
+// writes them (launch_after), so they are neither __restrict__ nor read by __ldg,
+// whose ld.global.nc needs memory that nobody writes while the grid lives; an
+// ordinary load after pdl_wait sees all that came before. The same goes for whatever
+// else a pass writes for the next: iterates and control blocks in the epilogues. The
+// matrix and its schedules, written by nothing between two passes, keep __ldg.
 template <class T, int NV>
 struct Gathers {
-    const T *__restrict__ p[NV];
+    const T *p[NV];
 };
+template <class T>
+__device__ __forceinline__ T gathered(const T *at) {
+    return *at;
+}
 
 // Epilogue interface (EpiBase has defaults for all but row_pre / row):
 //   static constexpr int NR;                            reduction slots (>= 1)
@@ -253,7 +263,7 @@ __global__ void __launch_bounds__(kTileThreads, MINB)
                     if (kb + 32 * u + lane < k1) {
 #pragma unroll
                         for (int q = 0; q < NV; ++q)
-                            part[q] += static_cast<A>(v[u]) * (gs[q] * static_cast<A>(__ldg(g.p[q] + c[u])));
+                            part[q] += static_cast<A>(v[u]) * (gs[q] * static_cast<A>(gathered(g.p[q] + c[u])));
                     }
                 }
             }
@@ -331,7 +341,7 @@ __global__ void __launch_bounds__(kTileThreads, MINB)
             for (int u = 0; u < U; ++u) {
                 const bool in = jb + 32 * u + lane < nz;
 #pragma unroll
-                for (int q = 0; q < NV; ++q) xv[q][u] = in ? static_cast<A>(__ldg(g.p[q] + c[u])) : A(0);
+                for (int q = 0; q < NV; ++q) xv[q][u] = in ? static_cast<A>(gathered(g.p[q] + c[u])) : A(0);
             }
             const int jn = jb + 32 * U;
             if (PIPE && jn < nz) {
@@ -432,7 +442,7 @@ __global__ void __launch_bounds__(kTileThreads, MINB)
                 if (kb + 32 * u + lane < k1) {
 #pragma unroll
                     for (int q = 0; q < NV; ++q)
-                        part[q] += static_cast<A>(v[u]) * (gs[q] * static_cast<A>(__ldg(g.p[q] + c[u])));
+                        part[q] += static_cast<A>(v[u]) * (gs[q] * static_cast<A>(gathered(g.p[q] + c[u])));
                 }
             }
         }
@@ -469,13 +479,13 @@ __global__ void __launch_bounds__(kTileThreads, MINB)
                 for (int u = 0; u < U; ++u)
 #pragma unroll
                     for (int q = 0; q < NV; ++q)
-                        part[q] += static_cast<A>(v[u]) * (gs[q] * static_cast<A>(__ldg(g.p[q] + c[u])));
+                        part[q] += static_cast<A>(v[u]) * (gs[q] * static_cast<A>(gathered(g.p[q] + c[u])));
             }
             for (; k < b; k += L) {
                 const int c = __ldg(M.ci + k);
                 const A v = static_cast<A>(__ldg(M.val + k));
 #pragma unroll
-                for (int q = 0; q < NV; ++q) part[q] += v * (gs[q] * static_cast<A>(__ldg(g.p[q] + c)));
+                for (int q = 0; q < NV; ++q) part[q] += v * (gs[q] * static_cast<A>(gathered(g.p[q] + c)));
             }
 #pragma unroll
             for (int o = L / 2; o > 0; o >>= 1)
@@ -592,7 +602,7 @@ __global__ void __launch_bounds__(kTileThreads, MINB)
                 if (u < len) {
 #pragma unroll
                     for (int q = 0; q < NV; ++q)
-                        sum[q] += static_cast<A>(v[u]) * (gs[q] * static_cast<A>(__ldg(g.p[q] + c[u])));
+                        sum[q] += static_cast<A>(v[u]) * (gs[q] * static_cast<A>(gathered(g.p[q] + c[u])));
                 }
         }
         unsigned lm = __ballot_sync(FULL, valid && len > S);
@@ -618,7 +628,7 @@ __global__ void __launch_bounds__(kTileThreads, MINB)
                         if (kb + 32 * u + lane < fb) {
 #pragma unroll
                             for (int q = 0; q < NV; ++q)
-                                part[q] += static_cast<A>(v[u]) * (gs[q] * static_cast<A>(__ldg(g.p[q] + c[u])));
+                                part[q] += static_cast<A>(v[u]) * (gs[q] * static_cast<A>(gathered(g.p[q] + c[u])));
                         }
                 }
 #pragma unroll
@@ -652,7 +662,7 @@ __global__ void __launch_bounds__(kTileThreads, MINB)
                         if (kb + u * L < rz) {
 #pragma unroll
                             for (int q = 0; q < NV; ++q)
-                                part[q] += static_cast<A>(v[u]) * (gs[q] * static_cast<A>(__ldg(g.p[q] + c[u])));
+                                part[q] += static_cast<A>(v[u]) * (gs[q] * static_cast<A>(gathered(g.p[q] + c[u])));
                         }
                 }
             }
@@ -771,7 +781,7 @@ __global__ void __launch_bounds__(kTileThreads, MINB)
 #pragma unroll
     for (int r = 0; r < NR; ++r) red[r] = 0.0;
     const A gs = epi.gscale(0);
-    const T *__restrict__ x = g.p[0];
+    const T *x = g.p[0];
 
     const int W = gridDim.x * kWarps;
     const int wid = blockIdx.x * kWarps + warp;
@@ -850,7 +860,7 @@ __global__ void __launch_bounds__(kTileThreads, MINB)
 #pragma unroll
             for (int u = 0; u < U; ++u) c[u] = j + 32 * u < nz ? sc[j + 32 * u] : 0;
 #pragma unroll
-            for (int u = 0; u < U; ++u) xv[u] = j + 32 * u < nz ? __ldg(x + c[u]) : T(0);
+            for (int u = 0; u < U; ++u) xv[u] = j + 32 * u < nz ? gathered(x + c[u]) : T(0);
 #pragma unroll
             for (int u = 0; u < U; ++u)
                 if (j + 32 * u < nz) sv[j + 32 * u] = static_cast<T>(static_cast<A>(sv[j + 32 * u]) * (gs * static_cast<A>(xv[u])));

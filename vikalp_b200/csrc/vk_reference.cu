@@ -188,7 +188,7 @@ struct RefColFastEpi : EpiBase<double> {
     __device__ bool skip() const { return ctl->done != 0; }
     __device__ Pre load(int j) const { return Pre{x[j], c[j], l[j], u[j], QP ? qx[j] : 0.0}; }
     __device__ void row_pre(int j, const double (&s)[1], const Pre &p, double (&red)[1]) const {
-        const long long k = __ldg(&ctl->iter);
+        const long long k = ctl->iter;
         const double g = QP ? __dadd_rn(s[0], __dadd_rn(p.c, p.qx)) : __dadd_rn(s[0], p.c);
         if (k >= 1) {
             const double px = clampbox(__dadd_rn(-g, p.x), p.l, p.u);
@@ -198,7 +198,7 @@ struct RefColFastEpi : EpiBase<double> {
             aty[j] = s[0];
             return;
         }
-        const double tau = __ldg(&ctl->tau);
+        const double tau = ctl->tau;
         xn[j] = QP ? clampbox(__dadd_rn(__dmul_rn(-tau, g), p.x), p.l, p.u)
                    : ref_primal(tau, s[0], p.x, p.c, p.l, p.u);
     }
