@@ -142,3 +142,28 @@ def test_instances_that_fit_one_sm_and_one_that_does_not():
         for k in want:
             if np.linalg.norm(want[k]) > 0:
                 assert rel(r[k], want[k]) <= 1e-8, (m, k, rel(r[k], want[k]))
+
+
+def test_gradients_do_not_depend_on_the_other_instances():
+    # a wide instance with few kept nonzeros (180 KB of vectors) and a narrow one
+    # with many (6,000, 120 KB): each fits one SM, one layout for both would not.
+    # The same bits alone, in either order and beside an instance that does not fit
+    # (2,000 x 8 kept); the reference point of both is the test above.
+    shapes = [(200, 15_000, 50, 3), (1000, 1500, 750, 8), (2500, 3500, 2000, 8)]
+    wide, narrow, large = [_planted(*s, seed=70 + k) for k, s in enumerate(shapes)]
+    rng = np.random.default_rng(3)
+    g = {id(i): rng.standard_normal(i[0].n) for i in (wide, narrow, large)}
+
+    def run(models):
+        return vk.lp_adjoint([t[0] for t in models], [t[1] for t in models], [t[2] for t in models],
+                             [g[id(t)] for t in models], 0.5, solve_tolerance=1e-12)
+
+    alone = {id(t): run([t])[0] for t in (wide, narrow)}
+    for models in ([wide, narrow], [narrow, wide], [wide, large, narrow]):
+        for t, r in zip(models, run(models)):
+            if t is large:
+                continue
+            want = alone[id(t)]
+            assert r["status"] == want["status"] == "Optimal" and r["iterations"] == want["iterations"]
+            for k in ("b", "A"):
+                assert np.array_equal(r[k], want[k]), (t[0].n, [u[0].n for u in models], k)

@@ -275,10 +275,12 @@ __global__ void adjoint_a_kernel(const int *__restrict__ ro, const int *__restri
 // shared memory and runs every iteration of its instance, with block barriers
 // in place of five launches an iteration: 64 LPs (m = 1,000, n = 2,000, 16,000
 // nonzeros, 3,900 of them active and free), 550 iterations, 55 -> 3 us each.
+// Whether an instance is solved so, and its layout, follow from its own sizes,
+// so that its gradients do not depend on the instances it is called with.
 constexpr int kAdjThreads = 1024;
 constexpr int kAdjSmem = 220 * 1024; // dynamic shared memory of a CTA (227 KB less the static part)
 
-// Sizes of one instance, or the largest of a launch.
+// Sizes of one instance; nnz: its kept nonzeros.
 struct AdjShape {
     int m = 0, n = 0, nnz = 0;
 };
@@ -412,17 +414,17 @@ struct AdjStep {
 // (AdjColEpi, AdjRowEpi, lsqr_*) with one reciprocal per scalar in place of a
 // division per element; thread 0 runs the scalar recurrences.
 __global__ void __launch_bounds__(kAdjThreads, 1)
-    adj_lsqr_kernel(LsqrCtl c, const int *__restrict__ list, const int *__restrict__ roff, const int *__restrict__ coff,
-                    const int *__restrict__ ro_a, const int *__restrict__ ci_a, const double *__restrict__ val_a,
-                    const int *__restrict__ ro_t, const int *__restrict__ ci_t, const double *__restrict__ val_t,
-                    const double *__restrict__ rmask, const double *__restrict__ fmask,
-                    const double *__restrict__ ubar, double *__restrict__ wout, AdjShape most) {
+    adj_lsqr_kernel(LsqrCtl c, const int *__restrict__ list, const int *__restrict__ kept,
+                    const int *__restrict__ roff, const int *__restrict__ coff, const int *__restrict__ ro_a,
+                    const int *__restrict__ ci_a, const double *__restrict__ val_a, const int *__restrict__ ro_t,
+                    const int *__restrict__ ci_t, const double *__restrict__ val_t, const double *__restrict__ rmask,
+                    const double *__restrict__ fmask, const double *__restrict__ ubar, double *__restrict__ wout) {
     extern __shared__ __align__(16) unsigned char adj_smem[];
     __shared__ double scratch[33];
     __shared__ int sums[32];
     const int b = list[blockIdx.x], tid = threadIdx.x;
     const int r0 = roff[b], m = roff[b + 1] - r0, c0 = coff[b], n = coff[b + 1] - c0;
-    const AdjLayout lay(most);
+    const AdjLayout lay(AdjShape{m, n, kept[b]});
     const auto vec = [&](size_t o) { return reinterpret_cast<double *>(adj_smem + o); };
     const auto ind = [&](size_t o) { return reinterpret_cast<uint16_t *>(adj_smem + o); };
     const auto off = [&](size_t o) { return reinterpret_cast<int *>(adj_smem + o); };
@@ -696,20 +698,20 @@ private:
         VK_CUDA(cudaMemcpyAsync(kept.data(), cnt.get(), cnt.bytes(), cudaMemcpyDeviceToHost, s_));
         VK_CUDA(cudaMemcpyAsync(roff.get(), h_.row_off.data(), roff.bytes(), cudaMemcpyHostToDevice, s_));
         VK_CUDA(cudaStreamSynchronize(s_));
-        AdjShape most;
+        size_t bytes = 0; // the largest instance's
         for (int b = 0; b < B; ++b) {
             const AdjShape s{h_.row_off[b + 1] - h_.row_off[b], h_.col_off[b + 1] - h_.col_off[b], kept[b]};
-            const AdjShape with{std::max(most.m, s.m), std::max(most.n, s.n), std::max(most.nnz, s.nnz)};
-            if (s.m == 0 || s.m > 65536 || s.n > 65536 || AdjLayout(with).bytes > static_cast<size_t>(kAdjSmem)) continue;
-            most = with;
+            const size_t own = AdjLayout(s).bytes;
+            if (s.m == 0 || s.m > 65536 || s.n > 65536 || own > static_cast<size_t>(kAdjSmem)) continue;
+            bytes = std::max(bytes, own);
             list.push_back(b);
         }
         if (list.empty()) return false;
         VK_CUDA(cudaMemcpyAsync(dlist.get(), list.data(), list.size() * sizeof(int), cudaMemcpyHostToDevice, s_));
         VK_CUDA(cudaFuncSetAttribute(adj_lsqr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAdjSmem));
-        adj_lsqr_kernel<<<static_cast<unsigned>(list.size()), kAdjThreads, AdjLayout(most).bytes, s_>>>(
-            c, dlist.get(), roff.get(), coff, d_.a.ro.get(), d_.a.ci.get(), d_.a_val.get(), d_.at.ro.get(),
-            d_.at.ci.get(), d_.at_val.get(), rmask_.get(), fmask_.get(), ubar_.get(), w_.get(), most);
+        adj_lsqr_kernel<<<static_cast<unsigned>(list.size()), kAdjThreads, bytes, s_>>>(
+            c, dlist.get(), cnt.get(), roff.get(), coff, d_.a.ro.get(), d_.a.ci.get(), d_.a_val.get(), d_.at.ro.get(),
+            d_.at.ci.get(), d_.at_val.get(), rmask_.get(), fmask_.get(), ubar_.get(), w_.get());
         VK_LAUNCH_CHECK();
         VK_CUDA(cudaStreamSynchronize(s_)); // the lists go out of scope
         return list.size() == static_cast<size_t>(B);
