@@ -41,8 +41,9 @@ struct Unsupported : std::runtime_error {
 // Device memory of the library's own solves (vk_pool.cu): a memory pool per
 // device, separate from the application's, that keeps up to kPoolKeep unused
 // bytes for the next call; the driver takes them back when an allocation of
-// the process needs them. A call on a batch makes ~200 allocations; cudaMalloc
-// and cudaFree took 5-25 ms of it, and up to a second when the host was busy.
+// the process needs them (another process can not have them). A call on a batch
+// makes ~200 allocations; cudaMalloc and cudaFree took 5-25 ms of it, and up to a
+// second when the host was busy.
 constexpr unsigned long long kPoolKeep = 2ull << 30;
 void *pool_alloc(size_t bytes, cudaStream_t s); // ordered on s
 void pool_free(void *p, cudaStream_t s) noexcept;
