@@ -272,7 +272,7 @@ inline void launch_after(K kernel, int grid, int threads, size_t smem, cudaStrea
 }
 
 // Codes a kernel writes to the device error flag (first one wins).
-enum DeviceError : int { kDevErrNone = 0, kDevErrBarrierTimeout = 1 };
+enum DeviceError : int { kDevErrNone = 0, kDevErrBarrierTimeout = 1, kDevErrGridTimeout = 2 };
 
 template <class T>
 __device__ __forceinline__ T warp_sum(T v) {

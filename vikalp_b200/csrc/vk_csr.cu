@@ -185,6 +185,7 @@ void check_device_error(cudaStream_t s) {
         VK_CUDA(cudaMemsetAsync(f, 0, sizeof(int), s));
         VK_CUDA(cudaStreamSynchronize(s));
         throw CudaFailure(h == kDevErrBarrierTimeout ? "a sparse pass timed out waiting for its staged tile"
+                          : h == kDevErrGridTimeout  ? "a resident solve timed out at a barrier of its blocks"
                                                      : "a kernel reported a device error");
     }
 }

@@ -194,10 +194,10 @@ __device__ __forceinline__ void rs_rows(const RsSide<T, I> &s, const A *prod, F 
     rs_rows(s, prod, [](int) { return 0; }, [&](int r, A sum, int) { row(r, sum); });
 }
 
-// A CTA's block barrier at the end of a gather: false when any of its threads
-// gave up (`ok` false), after recording that.
+// A CTA's block barrier at the end of a grid barrier: false when the thread that
+// waited gave up (`ok` false), after recording that.
 __device__ __forceinline__ bool rs_block(bool ok, int *err) {
-    if (!ok) atomicCAS(err, 0, static_cast<int>(kDevErrBarrierTimeout));
+    if (!ok) atomicCAS(err, 0, static_cast<int>(kDevErrGridTimeout));
     return __syncthreads_or(!ok) == 0;
 }
 
