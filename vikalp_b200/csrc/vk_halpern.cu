@@ -703,22 +703,30 @@ private:
     }
 
     // A model whose matrices fit the GPU's shared memory iterates there
-    // (vk_resident.cuh): 9.5 us an iteration against 23.7 for the passes at
-    // 600,000 nonzeros (float64), and, with the gathers still in row order, 16.1
-    // against 37.5 at 720,000 (past about 800,000 they no longer fit), 17.5
-    // against 26.4 at 940,000 (float32).
+    // (vk_resident.cuh), the smallest LPs in one cluster (vk_cluster.cuh); what
+    // neither takes keeps no plan. Resident against the passes, per iteration: 9.5
+    // us against 23.7 at 600,000 nonzeros (float64; past about 800,000 they no
+    // longer fit) and, timed with the gathers in row order, 17.5 against 26.4 at
+    // 940,000 (float32).
     void plan_resident() {
-        if (!rs_plan(dm_.a, dm_.at, dm_.qp ? &dm_.q : nullptr, plan_, s_)) return;
-        fits_resident<double>(rs64_, packed64_);
-        if (mixed_) fits_resident<float>(rs32_, packed32_);
-        partials_.reset(static_cast<size_t>(kRsMaxGrid) * kCheckSums);
-        // the smallest LPs: one cluster (vk_cluster.cuh)
-        if (dm_.qp || static_cast<size_t>(dm_.m + dm_.n) * sizeof(float) > kClVectorBytes ||
-            !rs_plan(dm_.a, dm_.at, nullptr, plan_cl_, s_, kClRanks))
+        const CsrPattern32 *q = dm_.qp ? &dm_.q : nullptr;
+        if (!dm_.qp && static_cast<size_t>(dm_.m + dm_.n) * sizeof(float) <= kClVectorBytes &&
+            rs_plan(dm_.a, dm_.at, nullptr, plan_cl_, s_, kClRanks)) {
+            plan_cl_.threads = cl_threads(dm_.nnz);
+            fits_cluster<double>(cl64_);
+            if (mixed_) fits_cluster<float>(cl32_);
+            if (!cl64_ && !cl32_) plan_cl_ = RsPlan();
+        }
+        if (cl64_ && (cl32_ || !mixed_)) return;
+        if (!rs_plan(dm_.a, dm_.at, q, plan_, s_)) return;
+        if (!cl64_) fits_resident<double>(rs64_, packed64_);
+        if (mixed_ && !cl32_) fits_resident<float>(rs32_, packed32_);
+        if (!rs64_ && !rs32_) {
+            plan_ = RsPlan();
             return;
-        plan_cl_.threads = cl_threads(dm_.nnz);
-        fits_cluster<double>(cl64_);
-        if (mixed_) fits_cluster<float>(cl32_);
+        }
+        if ((rs64_ && packed64_) || (rs32_ && packed32_)) rs_pack(dm_.a, dm_.at, q, plan_, s_);
+        partials_.reset(static_cast<size_t>(kRsMaxGrid) * kCheckSums);
     }
     template <class T>
     size_t cluster_layout() const {

@@ -287,8 +287,6 @@ std::unique_ptr<DeviceModel> upload_model(const vk_problem &p, cudaStream_t s, i
     up(dm->rl, p.row_lower, m);
     up(dm->ru, p.row_upper, m);
     dm->h_c.assign(p.c, p.c + n);
-    dm->h_vl.assign(p.var_lower, p.var_lower + n);
-    dm->h_vu.assign(p.var_upper, p.var_upper + n);
     VK_CUDA(cudaStreamSynchronize(s));
     return dm;
 }

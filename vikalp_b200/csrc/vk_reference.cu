@@ -555,6 +555,11 @@ private:
             });
             if (resident_ || !plan_.packed) break;
         }
+        if (!resident_) {
+            plan_ = RsPlan();
+            return;
+        }
+        if (plan_.packed) rs_pack(dm_.a, dm_.at, nullptr, plan_, s_);
         norms_.reset(8);
     }
     size_t cluster_layout() const {

@@ -106,13 +106,14 @@ bool rs_plan(const CsrPattern32 &a, const CsrPattern32 &at, const CsrPattern32 *
     constexpr int kCols = 1 << RsPacked::kColBits;
     const int most = std::max({plan.cap_a, plan.cap_t, plan.cap_q});
     plan.packed = ctas == 0 && m <= kCols && n <= kCols && most <= kRsPlaces;
-    if (plan.packed) {
-        pack(a, plan.part_a, plan.grid, plan.cap_a, plan.words_a, s);
-        pack(at, plan.part_t, plan.grid, plan.cap_t, plan.words_t, s);
-        if (q) pack(*q, plan.part_t, plan.grid, plan.cap_q, plan.words_q, s);
-    }
     VK_CUDA(cudaStreamSynchronize(s)); // the boundaries live on this stack frame
     return true;
+}
+
+void rs_pack(const CsrPattern32 &a, const CsrPattern32 &at, const CsrPattern32 *q, RsPlan &plan, cudaStream_t s) {
+    pack(a, plan.part_a, plan.grid, plan.cap_a, plan.words_a, s);
+    pack(at, plan.part_t, plan.grid, plan.cap_t, plan.words_t, s);
+    if (q) pack(*q, plan.part_t, plan.grid, plan.cap_q, plan.words_q, s);
 }
 
 int rs_grid(int64_t nnz) {

@@ -275,30 +275,26 @@ __device__ __forceinline__ bool rs_sum(double (&v)[NR], double *partials, double
 // The launch of a model: its shape, the largest shares, the shares' boundaries.
 struct RsPlan {
     bool small = false;  // 16-bit indices
-    bool packed = false; // gathers in column order (RsPacked)
+    bool packed = false; // gathers in column order (RsPacked): the bits can hold them
     int grid = 0, threads = 0;
     int cap_a = 0, cap_t = 0, cap_q = 0, rows = 0, cols = 0;
     DevBuf<int> part_a, part_t;
     DevBuf<unsigned> counter; // of the grid barrier
-    DevBuf<int> words_a, words_t, words_q; // packed: RsPacked, share by share
+    DevBuf<int> words_a, words_t, words_q; // rs_pack: RsPacked, share by share
     // the index array of a launch
     const int *index(const DevBuf<int> &words, const CsrPattern32 &p, bool use_packed) const {
         return use_packed ? words.get() : p.ci.get();
     }
 };
 
-// Fills `plan` for A, its transpose and (or null) Q; false when the matrices
-// can not fit in any precision, or a kernel variant is pinned.
-// `ctas`: that many shares (0: rs_grid's).
+// Fills `plan` for A, its transpose and (or null) Q, without the packed words;
+// false when the matrices can not fit in any precision, or a kernel variant is
+// pinned. `ctas`: that many shares (0: rs_grid's).
 bool rs_plan(const CsrPattern32 &a, const CsrPattern32 &at, const CsrPattern32 *q, RsPlan &plan, cudaStream_t s,
              int ctas = 0);
+// The packed words of a plan that a launch will use.
+void rs_pack(const CsrPattern32 &a, const CsrPattern32 &at, const CsrPattern32 *q, RsPlan &plan, cudaStream_t s);
 
-// CTAs (at most one per SM) and threads for `nnz` nonzeros. Timed per
-// iteration (float64 Halpern, 37 / 74 / 148 CTAs x 256 / 512 / 768 / 1024
-// threads): 4,000 nonzeros 4.6 us with 31 x 256 (148 x 1024: 5.3), 40,000
-// nonzeros 5.2 us with 148 x 256 (37 x 256: 6.5, 148 x 1024: 5.5), 120,000
-// nonzeros 6.0 us with 148 x 512 (256: 6.4, 1024: 6.5), 600,000 nonzeros 10.3
-// us with 148 x 768 (256: 12.2, 1024: 10.9).
 // f(a value of the index type of a launch): the plan's, or without its packing.
 template <class F>
 void rs_with_index(const RsPlan &plan, bool packed, F &&f) {
@@ -309,6 +305,12 @@ void rs_with_index(const RsPlan &plan, bool packed, F &&f) {
     else
         f(int());
 }
+// CTAs (at most one per SM) and threads for `nnz` nonzeros. Timed per
+// iteration (float64 Halpern, 37 / 74 / 148 CTAs x 256 / 512 / 768 / 1024
+// threads): 4,000 nonzeros 4.6 us with 31 x 256 (148 x 1024: 5.3), 40,000
+// nonzeros 5.2 us with 148 x 256 (37 x 256: 6.5, 148 x 1024: 5.5), 120,000
+// nonzeros 6.0 us with 148 x 512 (256: 6.4, 1024: 6.5), 600,000 nonzeros 10.3
+// us with 148 x 768 (256: 12.2, 1024: 10.9).
 int rs_grid(int64_t nnz);
 int rs_threads(int64_t nnz, int grid);
 

@@ -24,7 +24,6 @@ struct DeviceModel {
     std::vector<double> h_c;                 // for the host-side objective sum
     std::vector<int64_t> h_qro, h_qci;       // Q on the host (objective's quadratic term)
     std::vector<double> h_qv;
-    std::vector<double> h_vl, h_vu;          // model bounds (override validation)
     bool tuned = false;                      // pattern variants timed (ensure_tuned)
     // Column order (order_columns_by_count): when cperm is set, the device
     // side (a, at, a_val, at_val, c, vl, vu) is in the renamed order and
