@@ -679,15 +679,21 @@ private:
         return std::isfinite(o_.time_limit_seconds) && seconds_since(t0) >= o_.time_limit_seconds;
     }
 
-    // The next check interval (several in one launch of the float64 resident
-    // kernel: it stops by itself; the float32 phase's plateau rule wants every
-    // check, as does the trace), and the control block back on the host.
+    // The next check interval (several of the float64 resident kernel, which
+    // stops by itself, in launches of about kRsLaunch iterations; a cluster takes
+    // them in one; the float32 phase's plateau rule wants every check, as does
+    // the trace), and the control block back on the host.
     template <class T>
     void advance(HalState<T> &st, bool resident, cudaGraphExec_t g) {
         if (resident) {
-            const bool every = sizeof(T) == 4 || o_.verbose >= 2;
-            launch_resident(st, sizeof(T) == 4 ? cl32_ : cl64_, every ? 1 : std::max(1, kRsIterations / chunk_));
-            launches_ += 1;
+            const bool every = sizeof(T) == 4 || o_.verbose >= 2, cluster = sizeof(T) == 4 ? cl32_ : cl64_;
+            const int chunks = every ? 1 : std::max(1, (cluster ? kRsLook : kRsLaunch) / chunk_);
+            const long long left = (hctl_[0].limit - hctl_[0].total - 1) / chunk_ + 1; // checks to the limit
+            const long long most = every ? 1 : std::max<long long>(1, std::min<long long>(kRsLook / chunk_, left));
+            for (long long k = 0; k < most; k += chunks) {
+                launch_resident(st, cluster, chunks);
+                launches_ += 1;
+            }
         } else {
             VK_CUDA(cudaGraphLaunch(g, s_));
             launches_ += graph_nodes_;

@@ -446,7 +446,7 @@ public:
         VK_CUDA(cudaEventCreate(&e0));
         VK_CUDA(cudaEventCreate(&e1));
         VK_CUDA(cudaEventRecord(e0, s_));
-        for (long long k = 0; k < iterations; k += kRsIterations) launch_resident(cycles.get());
+        for (long long k = 0; k < iterations; k += iterations_per_launch()) launch_resident(cycles.get());
         VK_CUDA(cudaEventRecord(e1, s_));
         long long h[3];
         VK_CUDA(cudaMemcpyAsync(h, cycles.get(), sizeof(h), cudaMemcpyDeviceToHost, s_));
@@ -481,14 +481,19 @@ public:
         VK_CUDA(cudaEventCreate(&e1));
         VK_CUDA(cudaEventRecord(e0, s_));
         bool timed_out = false;
+        long long seen = 0; // iterations at the host's last look
         for (;;) {
             if (std::isfinite(o_.time_limit_seconds) && seconds_since(started) >= o_.time_limit_seconds) {
                 timed_out = true;
                 break;
             }
             if (resident_) {
-                launch_resident();
-                info.kernel_launches += 1;
+                // (the launch after the last iteration takes the stop)
+                const long long most = std::min<long long>(kRsLook - 1, o_.iteration_limit - seen);
+                for (long long k = 0; k <= most; k += iterations_per_launch()) {
+                    launch_resident();
+                    info.kernel_launches += 1;
+                }
             } else {
                 VK_CUDA(cudaGraphLaunch(graph_exec_, s_));
                 info.kernel_launches += graph_nodes_;
@@ -497,6 +502,7 @@ public:
             VK_CUDA(cudaStreamSynchronize(s_));
             check_device_error(s_);
             if (hctl_[0].done) break;
+            seen = hctl_[0].iter;
         }
         VK_CUDA(cudaEventRecord(e1, s_));
         VK_CUDA(cudaMemcpyAsync(hctl_.get(), ctl_.get(), sizeof(RefCtl), cudaMemcpyDeviceToHost, s_));
@@ -569,6 +575,7 @@ private:
     size_t layout() const {
         return RsRefLayout<I>(plan_.cap_a, plan_.cap_t, plan_.rows, plan_.cols).bytes;
     }
+    int iterations_per_launch() const { return cluster_ ? kRsLook : kRsLaunch; }
     void launch_resident(long long *cycles = nullptr) {
         RsRefArgs a{};
         a.cycles = cycles;
@@ -597,7 +604,7 @@ private:
         a.norms = norms_.get();
         a.counter = plan_.counter.get();
         a.err = device_error_flag();
-        a.iterations = kRsIterations;
+        a.iterations = iterations_per_launch();
         if (cluster_) {
             cl_reference_kernel<<<kClRanks, plan_.threads, cluster_layout(), s_>>>(a, dm_.m, dm_.n);
             VK_LAUNCH_CHECK();

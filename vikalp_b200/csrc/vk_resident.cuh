@@ -34,7 +34,13 @@ constexpr int kRsRowCost = 4;       // partition: a row costs this many nonzeros
 constexpr int kRsGather = 4;
 constexpr int kRsWarpRow = 32;      // a row of more than this many products per lane goes to a whole warp
 constexpr int kRsMaxGrid = 160;
-constexpr int kRsIterations = 1024; // iterations in one launch, about
+// Iterations in one launch, about: a launch holds the shared memory of every SM, and
+// other streams' kernels that need some wait for its end. A 2,048 x 2,048 bf16 product
+// beside solves of a 2,000 x 5,000 / 50,000 x 100,000 LP: 0.04-1.2 / 2.2 ms, with 1,024
+// iterations a launch 4.7 / 9.2 ms (alone 0.035); the solves themselves take 0.2-0.7%
+// longer (3.66 -> 3.69, 6.78 -> 6.81, 6.79 -> 6.81 ms).
+constexpr int kRsLaunch = 256;
+constexpr int kRsLook = 1024; // iterations between two looks of the host, about
 constexpr unsigned kRsPolls = 1u << 25; // over ten seconds
 
 // ---- device side ----------------------------------------------------------------
