@@ -710,10 +710,10 @@ private:
 
     // A model whose matrices fit the GPU's shared memory iterates there
     // (vk_resident.cuh), the smallest LPs in one cluster (vk_cluster.cuh); what
-    // neither takes keeps no plan. Resident against the passes, per iteration: 9.5
-    // us against 23.7 at 600,000 nonzeros (float64; past about 800,000 they no
-    // longer fit) and, timed with the gathers in row order, 17.5 against 26.4 at
-    // 940,000 (float32).
+    // neither takes keeps no plan. Resident against the passes with their best
+    // variant, us an iteration: 600,000 nonzeros 9.5 / 16.8, 720,000 13.3 / 17.7
+    // (float64; past about 800,000 they no longer fit), 936,000 in float32 with
+    // the float64 finish 11.6 / 20.4.
     void plan_resident() {
         const CsrPattern32 *q = dm_.qp ? &dm_.q : nullptr;
         if (!dm_.qp && static_cast<size_t>(dm_.m + dm_.n) * sizeof(float) <= kClVectorBytes &&
