@@ -410,15 +410,24 @@ struct AdjStep {
     int stop;
 };
 
+// Iterations in one launch: a CTA holds the shared memory of its SM while it lasts, and
+// other streams' kernels that need some wait for its end. A 2,048 x 2,048 bf16 product
+// beside 160 instances of 6,000 nonzeros with 100,000 iterations waited 541 ms for one
+// launch to the end; a launch of 1,024 takes 5 ms.
+constexpr int kAdjLaunch = 1024;
+
 // LSQR of instance list[blockIdx.x]: the steps of the pass kernels above
 // (AdjColEpi, AdjRowEpi, lsqr_*) with one reciprocal per scalar in place of a
-// division per element; thread 0 runs the scalar recurrences.
+// division per element; thread 0 runs the scalar recurrences. At most kAdjLaunch
+// iterations; an instance that needs more leaves its vectors and scalars as they
+// are and goes on from them when called with `resume`, to the same bits.
 __global__ void __launch_bounds__(kAdjThreads, 1)
     adj_lsqr_kernel(LsqrCtl c, const int *__restrict__ list, const int *__restrict__ kept,
                     const int *__restrict__ roff, const int *__restrict__ coff, const int *__restrict__ ro_a,
                     const int *__restrict__ ci_a, const double *__restrict__ val_a, const int *__restrict__ ro_t,
                     const int *__restrict__ ci_t, const double *__restrict__ val_t, const double *__restrict__ rmask,
-                    const double *__restrict__ fmask, const double *__restrict__ ubar, double *__restrict__ wout) {
+                    const double *__restrict__ fmask, bool resume, double *__restrict__ gu, double *__restrict__ gv,
+                    double *__restrict__ gw, double *__restrict__ gd) {
     extern __shared__ __align__(16) unsigned char adj_smem[];
     __shared__ double scratch[33];
     __shared__ int sums[32];
@@ -444,33 +453,52 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
     __shared__ AdjStep step;
     double beta = 0.0;
     for (int j = tid; j < n; j += kAdjThreads) {
-        ub[j] = ubar[c0 + j];
+        ub[j] = gu[c0 + j];
         beta += ub[j] * ub[j];
     }
-    for (int i = tid; i < m; i += kAdjThreads) w[i] = d[i] = vb[i] = 0.0;
+    for (int i = tid; i < m; i += kAdjThreads) {
+        vb[i] = resume ? gv[r0 + i] : 0.0;
+        w[i] = resume ? gw[r0 + i] : 0.0;
+        d[i] = resume ? gd[r0 + i] : 0.0;
+    }
     beta = sqrt(adj_sum(beta, scratch));
-    const double beta1 = beta;
-    double rnorm = beta, arnorm = 0.0, anorm2 = 0.0, phibar = beta, rhobar = 0.0, alpha = 0.0; // thread 0's
+    // thread 0's
+    double beta1 = beta, rnorm = beta, arnorm = 0.0, anorm2 = 0.0, phibar = beta, rhobar = 0.0, alpha = 0.0;
     long long iters = 0;
     int status = VK_STATUS_OPTIMAL; // g_F = 0, or orthogonal to the range of M: w = 0 is the answer
-    if (beta > 0.0) {
-        // v_1 = M'u_1 / beta_1, alpha_1 = |v_1|, d_1 = v_1
+    bool stopped = true;
+    if (beta > 0.0 || resume) {
         double sum = 0.0;
-        const double ibeta1 = 1.0 / beta;
-        adj_pass(va, ia, roa, m, la, ub, [&](int i, double s) {
-            vb[i] = s * ibeta1;
-            sum += vb[i] * vb[i];
-        });
-        sum = adj_sum(sum, scratch);
-        if (tid == 0) {
-            rhobar = alpha = sqrt(sum);
-            anorm2 = alpha * alpha;
-            arnorm = alpha * beta;
-            step = AdjStep{0.0, 0.0, alpha > 0.0 ? 1.0 / alpha : 0.0, alpha / beta, alpha > 0.0 ? 0 : 1};
+        if (resume) {
+            beta = c.beta[b];
+            if (tid == 0) {
+                beta1 = c.beta1[b];
+                alpha = c.alpha[b];
+                phibar = c.phibar[b];
+                rhobar = c.rhobar[b];
+                anorm2 = c.anorm2[b];
+                iters = c.iters[b];
+                step = AdjStep{0.0, 0.0, 1.0 / alpha, alpha * (beta > 0.0 ? 1.0 / beta : 0.0), 0};
+            }
+            __syncthreads();
+        } else {
+            // v_1 = M'u_1 / beta_1, alpha_1 = |v_1|, d_1 = v_1
+            const double ibeta1 = 1.0 / beta;
+            adj_pass(va, ia, roa, m, la, ub, [&](int i, double s) {
+                vb[i] = s * ibeta1;
+                sum += vb[i] * vb[i];
+            });
+            sum = adj_sum(sum, scratch);
+            if (tid == 0) {
+                rhobar = alpha = sqrt(sum);
+                anorm2 = alpha * alpha;
+                arnorm = alpha * beta;
+                step = AdjStep{0.0, 0.0, alpha > 0.0 ? 1.0 / alpha : 0.0, alpha / beta, alpha > 0.0 ? 0 : 1};
+            }
+            __syncthreads();
+            for (int i = tid; i < m; i += kAdjThreads) d[i] = vb[i] * step.ialpha;
         }
-        __syncthreads();
-        for (int i = tid; i < m; i += kAdjThreads) d[i] = vb[i] * step.ialpha;
-        while (!step.stop) {
+        for (int k = 0; k < kAdjLaunch && !step.stop; ++k) {
             const double ialpha = step.ialpha, wu = step.wv;
             sum = 0.0;
             adj_pass(vt, it, rot, n, lt, vb, [&](int j, double s) {
@@ -515,17 +543,33 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
                 d[i] = vb[i] * ia2 - t2 * di;
             }
         }
+        stopped = step.stop != 0;
     }
     __syncthreads();
-    for (int i = tid; i < m; i += kAdjThreads) wout[r0 + i] = w[i];
+    for (int i = tid; i < m; i += kAdjThreads) {
+        gw[r0 + i] = w[i];
+        if (!stopped) {
+            gv[r0 + i] = vb[i];
+            gd[r0 + i] = d[i];
+        }
+    }
+    if (!stopped)
+        for (int j = tid; j < n; j += kAdjThreads) gu[c0 + j] = ub[j];
     if (tid == 0) {
         c.beta1[b] = beta1;
         c.rnorm[b] = rnorm;
         c.arnorm[b] = arnorm;
         c.anorm2[b] = anorm2;
         c.iters[b] = iters;
-        c.status[b] = status;
-        c.stop[b] = c.done[b] = 1;
+        if (stopped) {
+            c.status[b] = status;
+            c.stop[b] = c.done[b] = 1;
+        } else { // from here on, at the next launch
+            c.alpha[b] = alpha;
+            c.beta[b] = beta;
+            c.phibar[b] = phibar;
+            c.rhobar[b] = rhobar;
+        }
     }
 }
 
@@ -707,14 +751,21 @@ private:
             list.push_back(b);
         }
         if (list.empty()) return false;
-        VK_CUDA(cudaMemcpyAsync(dlist.get(), list.data(), list.size() * sizeof(int), cudaMemcpyHostToDevice, s_));
         VK_CUDA(cudaFuncSetAttribute(adj_lsqr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAdjSmem));
-        adj_lsqr_kernel<<<static_cast<unsigned>(list.size()), kAdjThreads, bytes, s_>>>(
-            c, dlist.get(), cnt.get(), roff.get(), coff, d_.a.ro.get(), d_.a.ci.get(), d_.a_val.get(), d_.at.ro.get(),
-            d_.at.ci.get(), d_.at_val.get(), rmask_.get(), fmask_.get(), ubar_.get(), w_.get());
-        VK_LAUNCH_CHECK();
-        VK_CUDA(cudaStreamSynchronize(s_)); // the lists go out of scope
-        return list.size() == static_cast<size_t>(B);
+        const bool all = list.size() == static_cast<size_t>(B);
+        std::vector<int> stopped(B);
+        for (bool resume = false; !list.empty(); resume = true) {
+            VK_CUDA(cudaMemcpyAsync(dlist.get(), list.data(), list.size() * sizeof(int), cudaMemcpyHostToDevice, s_));
+            adj_lsqr_kernel<<<static_cast<unsigned>(list.size()), kAdjThreads, bytes, s_>>>(
+                c, dlist.get(), cnt.get(), roff.get(), coff, d_.a.ro.get(), d_.a.ci.get(), d_.a_val.get(),
+                d_.at.ro.get(), d_.at.ci.get(), d_.at_val.get(), rmask_.get(), fmask_.get(), resume, ubar_.get(),
+                vbar_.get(), w_.get(), dir_.get());
+            VK_LAUNCH_CHECK();
+            VK_CUDA(cudaMemcpyAsync(stopped.data(), stop_.get(), B * sizeof(int), cudaMemcpyDeviceToHost, s_));
+            VK_CUDA(cudaStreamSynchronize(s_)); // the lists are reused
+            list.erase(std::remove_if(list.begin(), list.end(), [&](int b) { return stopped[b] != 0; }), list.end());
+        }
+        return all;
     }
 
     void row_pass(const LsqrCtl &c) {
